@@ -436,10 +436,12 @@ int fsl_trainer_get_weights(fsl_trainer *t, float *params)
 int fsl_trainer_set_weights(fsl_trainer *t, const float *params)
 {
     if (!t || !params) return FSL_ERR_ARG;
-    if (cudaMemcpy(t->P, params, kNParams * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+    // on the trainer's own stream, which the passes queued after it follow
+    if (cudaMemcpyAsync(t->P, params, kNParams * sizeof(float), cudaMemcpyHostToDevice, t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->M, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->V, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
+        cudaStreamSynchronize(t->st) != cudaSuccess)
         return FSL_ERR_CUDA;
-    cudaMemset(t->M, 0, kNParams * sizeof(float));
-    cudaMemset(t->V, 0, kNParams * sizeof(float));
     t->adam_t = 0;
     return FSL_OK;
 }
@@ -461,7 +463,10 @@ static int trainer_weights(fsl_trainer *t)
     return FSL_OK;
 }
 
-static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long long n, float lr, double *loss)
+// One gradient (lr 0) or Adam pass.  With wait the host reads the loss and the
+// error flag; without, the pass is only queued: a pass that gives up sets the
+// flag, the passes after it do nothing, and the next waiting pass reports it.
+static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long long n, float lr, double *loss, bool wait)
 {
     if (trainer_weights(t)) return FSL_ERR_CUDA;
     const float iw = t->loss_mode ? t->inv_wmean : 0.f;
@@ -475,7 +480,8 @@ static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long lon
         b1t = (float)std::pow(0.9, (double)t->adam_t);
         b2t = (float)std::pow(0.999, (double)t->adam_t);
     }
-    launch_reduce_adam(t->st, t->Gpart, nblk, t->P, t->M, t->V, t->Gout, lr, b1t, b2t);
+    launch_reduce_adam(t->st, t->Gpart, nblk, t->P, t->M, t->V, t->Gout, lr, b1t, b2t, t->err);
+    if (!wait) return FSL_OK;
     if (loss) {
         std::vector<float> lp(nblk);
         if (cudaMemcpyAsync(lp.data(), t->lossp, nblk * sizeof(float), cudaMemcpyDeviceToHost, t->st) !=
@@ -495,7 +501,7 @@ static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long lon
 int fsl_trainer_gradient(fsl_trainer *t, long long n, float *grad, double *loss)
 {
     if (!t || n < 1 || n > t->n) return FSL_ERR_ARG;
-    int rc = trainer_pass(t, t->X, t->Y, n, 0.f, loss);
+    int rc = trainer_pass(t, t->X, t->Y, n, 0.f, loss, true);
     if (rc) return rc;
     if (grad && cudaMemcpy(grad, t->Gout, kNParams * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
         return FSL_ERR_CUDA;
@@ -521,7 +527,7 @@ int fsl_trainer_train(fsl_trainer *t, int epochs, long long batch, double lr, do
     const long long nb = t->n / batch;
     for (int e = 0; e < epochs; e++)
         for (long long b = 0; b < nb; b++) {
-            int rc = trainer_pass(t, t->X + b * batch * 8, t->Y + b * batch, batch, (float)lr, nullptr);
+            int rc = trainer_pass(t, t->X + b * batch * 8, t->Y + b * batch, batch, (float)lr, nullptr, false);
             if (rc) return rc;
         }
     return fsl_trainer_gradient(t, t->n, nullptr, loss);

@@ -482,10 +482,8 @@ struct SmemTrain {
     alignas(128) __nv_bfloat16 A2T[64 * 128];
     alignas(128) __nv_bfloat16 DZ[128 * 64];   // dz, [cell][out]
     alignas(128) __nv_bfloat16 DZT[128 * 128]; // dz, [out (64, zero-padded to 128)][cell]
-    float gb[3 * 64];                // bias gradients b1 b2 b3
-    float gw4[64];
-    float gb4;
-    float loss;
+    float gsum[4][4][64];            // per warp: the gradients of b1, b2, b3, w4
+    float gone[4][2];                // per warp: the gradient of b4, the loss
     uint64_t mbar;
     uint32_t tholder;
 };
@@ -506,10 +504,72 @@ __device__ __forceinline__ void sync_for_mma()
     umma::fence_after_sync();
 }
 
+// 16 consecutive columns (from column c0, a multiple of 8) of row t of a K-major
+// tile of width 64, as two 16-byte stores.
+__device__ __forceinline__ void store_row16(__nv_bfloat16 *A, int t, int c0, const float *v)
+{
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t p[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[8 * h + 2 * q], v[8 * h + 2 * q + 1]);
+            p[q] = *reinterpret_cast<const uint32_t *>(&b);
+        }
+        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(A) + umma::tile_off(t, c0 + 8 * h, 64)) =
+            make_uint4(p[0], p[1], p[2], p[3]);
+    }
+}
+
+// This warp's 32 rows of the 128 x 64 tile A (K-major, width 64) into the
+// transposed tile AT (rows = A's columns, width 128): 8 x 8 core matrices
+// through ldmatrix.trans / stmatrix, four at a time.
+__device__ __forceinline__ void transpose_rows(const __nv_bfloat16 *A, __nv_bfloat16 *AT, int wp, int l)
+{
+    __syncwarp();
+    const uint32_t src = umma::smem_u32(A) + (uint32_t)(wp * 4 + (l >> 3)) * 1024u + (uint32_t)(l & 7) * 16u;
+    const uint32_t dst = umma::smem_u32(AT) + (uint32_t)(wp * 4 + (l >> 3)) * 128u + (uint32_t)(l & 7) * 16u;
+#pragma unroll
+    for (uint32_t ob = 0; ob < 8; ob++) {
+        uint32_t r0, r1, r2, r3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                     : "r"(src + ob * 128u)
+                     : "memory");
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + ob * 2048u), "r"(r0),
+                     "r"(r1), "r"(r2), "r"(r3)
+                     : "memory");
+    }
+}
+
+// Sums over the warp's lanes of 16 values per lane: lane l receives the sum of
+// value l & 15 (a halving butterfly: 16 shuffles instead of 16 x 5).
+__device__ __forceinline__ float warp_colsum16(const float *in, int l)
+{
+    float v[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = in[q];
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool up = (l & h) != 0;
+#pragma unroll
+        for (int q = 0; q < h; q++) {
+            const float give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
 // Gradient of the mean squared error over n samples for the parameters P,
 // accumulated per block into Gpart[blockIdx.x][kNParams]; loss_part holds
 // the block's summed squared error.  Each block handles tiles
-// [blockIdx.x * tpb, (blockIdx.x + 1) * tpb).
+// [blockIdx.x * tpb, (blockIdx.x + 1) * tpb).  TMEM (448 of 512 columns) allows
+// one block of four warps per SM, so the chain of seven products and their
+// epilogues bounds it.  The bias, w4 and loss sums are taken over a warp's
+// lanes with shuffles and kept in registers from tile to tile: as atomic adds
+// to one shared word per column they serialised a tile's 128 threads 256
+// times over (a gradient of 2^20 samples: 75 ms then, 0.85 ms now).
 __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__ X, const float *__restrict__ Yt,
                                                        long long n, int tpb, const float *__restrict__ P,
                                                        float *__restrict__ Gpart, float *__restrict__ loss_part,
@@ -517,17 +577,19 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     SmemTrain &s = *reinterpret_cast<SmemTrain *>(smraw);
-    const int t = threadIdx.x, wp = t >> 5;
+    if (*err) return; // an earlier pass gave up: its caller reports it
+    const int t = threadIdx.x, wp = t >> 5, l = t & 31;
     stage_weights(s.w, P, t, 128);
     for (int e = t; e < 64 * 64; e += 128) {
         const int o = e / 64, i = e % 64; // W[o][i] -> WT[i][o]
         s.W2T[umma::tile_off(i, o, 64) / 2] = __float2bfloat16_rn(P[kOffW2 + e]);
         s.W3T[umma::tile_off(i, o, 64) / 2] = __float2bfloat16_rn(P[kOffW3 + e]);
     }
+    // the padding: rows 64..127 of dz^T, inputs 8..15 of the features
     for (int e = t; e < 128 * 128; e += 128) s.DZT[e] = __float2bfloat16_rn(0.f);
-    for (int e = t; e < 3 * 64; e += 128) s.gb[e] = 0.f;
-    if (t < 64) s.gw4[t] = 0.f;
-    if (t == 0) { s.gb4 = 0.f; s.loss = 0.f; umma::mbar_init(&s.mbar, 1); }
+    for (int e = t; e < 128 * 16; e += 128) s.A0[e] = s.A0T[e] = __float2bfloat16_rn(0.f);
+    if (t == 0) umma::mbar_init(&s.mbar, 1);
+    float gb1[4] = {}, gb2[4] = {}, gb3[4] = {}, gw4[4] = {}, gb4 = 0.f, loss = 0.f;
     if (wp == 0) umma::tmem_alloc(&s.tholder, 512);
     umma::fence_before_sync();
     __syncthreads();
@@ -543,55 +605,68 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
     uint32_t phase = 0;
     bool ok = true;
     const long long ntile = (n + 127) / 128;
+    float4 x0, x1; // the sample of this thread (each is 32 bytes, so 16-byte aligned)
+    float yt;
+    auto fetch = [&](long long tile, bool more) {
+        const long long m = tile * 128 + t;
+        x0 = x1 = make_float4(0.f, 0.f, 0.f, 0.f);
+        yt = 0.f;
+        if (more && m < n) {
+            x0 = reinterpret_cast<const float4 *>(X)[2 * m];
+            x1 = reinterpret_cast<const float4 *>(X)[2 * m + 1];
+            yt = Yt[m];
+        }
+    };
+    fetch((long long)blockIdx.x * tpb, true);
     for (int tt = 0; tt < tpb && ok; tt++) {
         const long long tile = (long long)blockIdx.x * tpb + tt;
         if (tile >= ntile) break; // uniform across the block
         const bool acc = tt > 0;
-        const long long m = tile * 128 + t;
-        const bool valid = m < n;
-        float f[8];
+        const bool valid = tile * 128 + t < n;
+        const float f[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+        const float target = yt;
+        fetch(tile + 1, tt + 1 < tpb); // the next tile's samples, in flight during this one
+        {
+            uint32_t p[4];
 #pragma unroll
-        for (int q = 0; q < 8; q++) f[q] = valid ? X[m * 8 + q] : 0.f;
-        const float target = valid ? Yt[m] : 0.f;
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const __nv_bfloat16 b = __float2bfloat16_rn(q < 8 ? f[q] : 0.f);
-            s.A0[umma::tile_off(t, q, 16) / 2] = b;
-            s.A0T[umma::tile_off(q, t, 128) / 2] = b;
+            for (int q = 0; q < 4; q++) {
+                const __nv_bfloat162 b = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+                p[q] = *reinterpret_cast<const uint32_t *>(&b);
+                s.A0T[umma::tile_off(2 * q, t, 128) / 2] = __low2bfloat16(b);
+                s.A0T[umma::tile_off(2 * q + 1, t, 128) / 2] = __high2bfloat16(b);
+            }
+            *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(s.A0) + umma::tile_off(t, 0, 16)) =
+                make_uint4(p[0], p[1], p[2], p[3]);
         }
         // ---- forward: z1, z2, z3 stay in TMEM ----
         sync_for_mma();
         if (t == 0) { umma::gemm_issue(tmem + kZ1, aA0, aW1, 16, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
         if (!ok) break;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
             float v[16];
             umma::tmem_ld16(lane + kZ1 + c * 16, v);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int o = c * 16 + q;
-                const __nv_bfloat16 b = __float2bfloat16_rn(silu(v[q] + s.w.b1[o]));
-                s.A1[umma::tile_off(t, o, 64) / 2] = b;
-                s.A1T[umma::tile_off(o, t, 128) / 2] = b;
-            }
+            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b1[c * 16 + q]);
+            store_row16(s.A1, t, c * 16, v);
         }
+        transpose_rows(s.A1, s.A1T, wp, l);
         sync_for_mma();
         if (t == 0) { umma::gemm_issue(tmem + kZ2, aA1, aW2, 64, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
         if (!ok) break;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
             float v[16];
             umma::tmem_ld16(lane + kZ2 + c * 16, v);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int o = c * 16 + q;
-                const __nv_bfloat16 b = __float2bfloat16_rn(silu(v[q] + s.w.b2[o]));
-                s.A2[umma::tile_off(t, o, 64) / 2] = b;
-                s.A2T[umma::tile_off(o, t, 128) / 2] = b;
-            }
+            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b2[c * 16 + q]);
+            store_row16(s.A2, t, c * 16, v);
         }
+        transpose_rows(s.A2, s.A2T, wp, l);
         sync_for_mma();
         if (t == 0) { umma::gemm_issue(tmem + kZ3, aA2, aW3, 64, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
@@ -599,6 +674,7 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         // ---- output, loss gradient, layer 3 backward ----
         float z3[64];
         float y = s.w.b4;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
             float v[16];
             umma::tmem_ld16(lane + kZ3 + c * 16, v);
@@ -619,17 +695,22 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         }
         const float e = valid ? (y - target) : 0.f;
         const float dy = scale * wgt * e;
-        atomicAdd(&s.loss, wgt * e * e);
-        atomicAdd(&s.gb4, dy);
+        loss += wgt * e * e;
+        gb4 += dy;
 #pragma unroll
-        for (int o = 0; o < 64; o++) {
-            atomicAdd(&s.gw4[o], dy * silu(z3[o]));
-            const float dz = dy * s.w.w4[o] * dsilu(z3[o]);
-            atomicAdd(&s.gb[128 + o], dz);
-            const __nv_bfloat16 b = __float2bfloat16_rn(dz);
-            s.DZ[umma::tile_off(t, o, 64) / 2] = b;
-            s.DZT[umma::tile_off(o, t, 128) / 2] = b;
+        for (int c = 0; c < 4; c++) {
+            float v[16], g4[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float z = z3[c * 16 + q];
+                g4[q] = dy * silu(z);
+                v[q] = dy * s.w.w4[c * 16 + q] * dsilu(z);
+            }
+            gw4[c] += warp_colsum16(g4, l);
+            gb3[c] += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c * 16, v);
         }
+        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW3 += dz3^T a2 ; da2 = dz3 W3
         sync_for_mma();
         if (t == 0) {
@@ -639,21 +720,18 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         }
         mma_wait(s, phase, ok);
         if (!ok) break;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
             float v[16], zz[16];
             umma::tmem_ld16(lane + kDG + c * 16, v);
             umma::tmem_ld16(lane + kZ2 + c * 16, zz);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int o = c * 16 + q;
-                const float dz = valid ? v[q] * dsilu(zz[q] + s.w.b2[o]) : 0.f;
-                atomicAdd(&s.gb[64 + o], dz);
-                const __nv_bfloat16 b = __float2bfloat16_rn(dz);
-                s.DZ[umma::tile_off(t, o, 64) / 2] = b;
-                s.DZT[umma::tile_off(o, t, 128) / 2] = b;
-            }
+            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b2[c * 16 + q]) : 0.f;
+            gb2[c] += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c * 16, v);
         }
+        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW2 += dz2^T a1 ; da1 = dz2 W2
         sync_for_mma();
         if (t == 0) {
@@ -663,19 +741,18 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         }
         mma_wait(s, phase, ok);
         if (!ok) break;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
             float v[16], zz[16];
             umma::tmem_ld16(lane + kDG + c * 16, v);
             umma::tmem_ld16(lane + kZ1 + c * 16, zz);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int o = c * 16 + q;
-                const float dz = valid ? v[q] * dsilu(zz[q] + s.w.b1[o]) : 0.f;
-                atomicAdd(&s.gb[o], dz);
-                s.DZT[umma::tile_off(o, t, 128) / 2] = __float2bfloat16_rn(dz);
-            }
+            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b1[c * 16 + q]) : 0.f;
+            gb1[c] += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c * 16, v);
         }
+        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW1 += dz1^T a0
         sync_for_mma();
         if (t == 0) {
@@ -685,6 +762,22 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         mma_wait(s, phase, ok);
         if (!ok) break;
     }
+    // the warps' sums to shared memory (lanes 0..15 hold a chunk's 16 columns)
+    if (l < 16) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            s.gsum[wp][0][c * 16 + l] = gb1[c];
+            s.gsum[wp][1][c * 16 + l] = gb2[c];
+            s.gsum[wp][2][c * 16 + l] = gb3[c];
+            s.gsum[wp][3][c * 16 + l] = gw4[c];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
+    }
+    if (l == 0) { s.gone[wp][0] = gb4; s.gone[wp][1] = loss; }
     // ---- block partial gradients ----
     float *G = Gpart + (long long)blockIdx.x * kNParams;
     if (ok) {
@@ -705,15 +798,14 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
             for (int q = 0; q < 16; q++) G[kOffW1 + o * 16 + q] = (q < 8) ? v[q] : 0.f;
         }
         __syncthreads();
-        if (t < 64) {
-            G[kOffB1 + t] = s.gb[t];
-            G[kOffB2 + t] = s.gb[64 + t];
-            G[kOffB3 + t] = s.gb[128 + t];
-            G[kOffW4 + t] = s.gw4[t];
+        for (int e = t; e < 4 * 64; e += 128) {
+            const int which = e >> 6, o = e & 63;
+            const int at = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
+            G[at + o] = s.gsum[0][which][o] + s.gsum[1][which][o] + s.gsum[2][which][o] + s.gsum[3][which][o];
         }
         if (t == 0) {
-            G[kOffB4] = s.gb4;
-            loss_part[blockIdx.x] = s.loss;
+            G[kOffB4] = s.gone[0][0] + s.gone[1][0] + s.gone[2][0] + s.gone[3][0];
+            loss_part[blockIdx.x] = s.gone[0][1] + s.gone[1][1] + s.gone[2][1] + s.gone[3][1];
         }
     } else {
         if (t == 0) atomicExch(err, 1);
@@ -724,15 +816,24 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
     if (wp == 0) umma::tmem_free(tmem, 512);
 }
 
-// Deterministic sum of the block partials and an Adam step (FP32 master weights).
+// Deterministic sum of the block partials and an Adam step (FP32 master
+// weights); no step after a pass that gave up.  The partials are read eight
+// at a time (a serial chain of loads per parameter otherwise) and added in
+// block order.
 __global__ void k_reduce_adam(const float *__restrict__ Gpart, int nblk, float *__restrict__ P,
                               float *__restrict__ Mo, float *__restrict__ Vo, float *__restrict__ Gout, float lr,
-                              float b1t, float b2t)
+                              float b1t, float b2t, const int *err)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kNParams) return;
+    if (p >= kNParams || *err) return;
     float g = 0.f;
-    for (int b = 0; b < nblk; b++) g += Gpart[(long long)b * kNParams + p];
+    for (int b = 0; b < nblk; b += 8) {
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = b + q < nblk ? Gpart[(long long)(b + q) * kNParams + p] : 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; q++) g += v[q];
+    }
     if (Gout) Gout[p] = g;
     if (lr <= 0.f) return;
     const bool padded = (p >= kOffW1 && p < kOffW1 + 64 * 16 && ((p - kOffW1) % 16) >= 8);
@@ -825,9 +926,9 @@ int launch_train_grad(cudaStream_t st, const float *X, const float *Y, long long
 }
 
 void launch_reduce_adam(cudaStream_t st, const float *Gpart, int nblk, float *P, float *M, float *V, float *Gout,
-                        float lr, float b1t, float b2t)
+                        float lr, float b1t, float b2t, const int *err)
 {
-    mlp::k_reduce_adam<<<(kNParams + 255) / 256, 256, 0, st>>>(Gpart, nblk, P, M, V, Gout, lr, b1t, b2t);
+    mlp::k_reduce_adam<<<(kNParams + 63) / 64, 64, 0, st>>>(Gpart, nblk, P, M, V, Gout, lr, b1t, b2t, err);
 }
 
 namespace {
