@@ -14,7 +14,9 @@
 //    primitives twice (y/z sweeps of plane i, x sweep of plane i+1), the
 //    three sweeps, one velocity set of each form and one face viscosity
 //    average per cell (shared by the faces through on-chip memory), three
-//    face fluxes, the same combination.  The plain FP64 kernel.
+//    face fluxes, the same combination.  The plain FP64 method in the
+//    reference's expressions (its kernel forms the primitives once and takes
+//    the limiter in pairs, for the same values).
 //  * "fused_fp32": the same with the FP32 bulk's regrouped sweeps and paired
 //    limiter (recon_sweep_grouped, minmod2).
 // Sign flips and absolute values are operand modifiers and are not counted;

@@ -168,6 +168,11 @@ template <typename T, int TJE, bool PPM = false> struct Smem {
     T Dv[2][TJE][32][5];    // velocities by division, temperature, mu face average, planes i, i+1
     T Lo[TJE][32][5];       // y sweep: state on the face below each cell
     T Fy[TJE][32][5];       // y flux on the face above each row
+    // FP64: sound speed, 1/(2C) and 1/(2C)/C of planes i, i+1 (with R the roots
+    // of the cell's characteristic transform), formed once per cell instead of
+    // by the y and z sweeps and again by the x sweep a plane earlier
+    static constexpr bool ROOTS = sizeof(T) == 8;
+    T C[2][ROOTS ? TJE : 1][32][3];
 };
 
 template <typename T> struct Args {
@@ -257,12 +262,39 @@ __device__ __forceinline__ void plane_prims(Smem<T, TJE, PPM> &s, int pl, int r,
 {
     constexpr int HW = Smem<T, TJE, PPM>::HW, NS = Smem<T, TJE, PPM>::NS;
     const T *u = s.U[pl & (NS - 1)][r + HW][l + HW];
-    vel_rcp(u[0], u[1], u[2], u[3], s.R[pl % 3][r][l]);
+    if constexpr (Smem<T, TJE, PPM>::ROOTS) {
+        CellC<T> c;
+#pragma unroll
+        for (int q = 0; q < 5; q++) c.u[q] = u[q];
+        cell_roots(c); // U, V, W are the reciprocal velocities of vel_rcp
+        T *v = s.R[pl % 3][r][l], *k = s.C[pl & 1][r][l];
+        v[0] = c.U; v[1] = c.V; v[2] = c.W;
+        k[0] = c.C; k[1] = c.ll; k[2] = c.ee;
+    } else {
+        vel_rcp(u[0], u[1], u[2], u[3], s.R[pl % 3][r][l]);
+    }
     T dv[4];
     vdiv(u, dv);
     T *o = s.Dv[pl & 1][r][l];
     o[0] = dv[0]; o[1] = dv[1]; o[2] = dv[2]; o[3] = dv[3];
     if constexpr (!SST) o[4] = T(0.5) * (mu_pl + mu_prev);
+}
+
+// The characteristic transform of the own cell of plane `pl` (state cell u),
+// from the stored roots or from the state.
+template <typename T, int TJE, bool PPM>
+__device__ __forceinline__ void ring_consts(const Smem<T, TJE, PPM> &s, const T *u, int pl, int r, int l, CellC<T> &c)
+{
+#pragma unroll
+    for (int q = 0; q < 5; q++) c.u[q] = u[q];
+    if constexpr (Smem<T, TJE, PPM>::ROOTS) {
+        const T *v = s.R[pl % 3][r][l], *k = s.C[pl & 1][r][l];
+        c.U = v[0]; c.V = v[1]; c.W = v[2];
+        c.C = k[0]; c.ll = k[1]; c.ee = k[2];
+        cell_products(c);
+    } else {
+        cell_consts(c);
+    }
 }
 
 // SST: static Smagorinsky (the face viscosity from the face gradients and the
@@ -405,10 +437,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
             const bool rz = zrow && k >= 1 && k <= D;
             if (ry || rz) {
                 CellC<T> cc;
-                const T *Uc = s.U[q0][r + HW][l + HW];
-#pragma unroll
-                for (int q = 0; q < 5; q++) cc.u[q] = Uc[q];
-                cell_consts(cc);
+                ring_consts<T, TJE, PPM>(s, s.U[q0][r + HW][l + HW], i, r, l, cc);
                 T fw[5], bw[5], lo[5];
                 if (ry) {
                     const T *a1 = s.U[q0][r + HW + 1][l + HW], *b1 = s.U[q0][r + HW - 1][l + HW];
@@ -500,10 +529,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
             T lo[5];
             if (i + 1 <= L) {
                 CellC<T> cc;
-                const T *Un = s.U[q1][r + HW][l + HW];
-#pragma unroll
-                for (int q = 0; q < 5; q++) cc.u[q] = Un[q];
-                cell_consts(cc);
+                ring_consts<T, TJE, PPM>(s, s.U[q1][r + HW][l + HW], i + 1, r, l, cc);
                 if constexpr (PPM) {
                     // planes i-1 .. i+2 from the ring (own column), i+3 in flight
                     const T *Um1 = s.U[(i - 1) & (NS - 1)][r + HW][l + HW], *U0 = s.U[q0][r + HW][l + HW];
