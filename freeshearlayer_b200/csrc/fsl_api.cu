@@ -125,19 +125,6 @@ int ensure_faces(Ctx &c)
     return FSL_OK;
 }
 
-int ensure_dyn(Ctx &c)
-{
-    if (c.dyn_alloc) return FSL_OK;
-    const size_t fs = (size_t)c.g.fstride;
-    int rc;
-    if ((rc = dev_alloc(c, &c.dyn.vel, 3 * fs))) return rc;
-    if ((rc = dev_alloc(c, &c.dyn.F, 9 * fs))) return rc;
-    if ((rc = dev_alloc(c, &c.dyn.A, 6 * fs))) return rc;
-    if ((rc = dev_alloc(c, &c.dyn.S, fs))) return rc;
-    c.dyn_alloc = true;
-    return FSL_OK;
-}
-
 int ensure_bf(Ctx &c)
 {
     if (c.bf_alloc) return FSL_OK;
@@ -180,11 +167,6 @@ int ensure_fp32(Ctx &c)
     if ((rc = dev_alloc_f(c, &c.bf32.z0, nz))) return rc;
     if ((rc = dev_alloc_f(c, &c.bf32.zD, nz))) return rc;
     if ((rc = dev_alloc_f(c, &c.mu32, (size_t)g.fstride))) return rc;
-    const size_t fs = (size_t)g.fstride;
-    if ((rc = dev_alloc_f(c, &c.dyn32.vel, 3 * fs))) return rc;
-    if ((rc = dev_alloc_f(c, &c.dyn32.F, 9 * fs))) return rc;
-    if ((rc = dev_alloc_f(c, &c.dyn32.A, 6 * fs))) return rc;
-    if ((rc = dev_alloc_f(c, &c.dyn32.S, fs))) return rc;
     c.fp32_alloc = true;
     return FSL_OK;
 }
@@ -194,13 +176,11 @@ double *cur_ptr(Ctx &c) { return c.cur ? c.Up : c.U; }
 } // namespace
 
 namespace fsl {
-int ensure_dyn_scratch(Ctx &c)
+int ensure_sgs(Ctx &c)
 {
-    // the dynamic procedure's scratch and, on the FP32 path, the FP32 SGS
-    // field it writes (allocated on first use, like the fused step's buffers)
-    int rc = ensure_dyn(c);
-    if (!rc && c.p.precision == FSL_PREC_FP32) rc = ensure_fp32(c);
-    return rc;
+    // the FP32 SGS field the dynamic procedure writes on the FP32 path
+    // (allocated on first use, like the fused step's buffers)
+    return c.p.precision == FSL_PREC_FP32 ? ensure_fp32(c) : FSL_OK;
 }
 } // namespace fsl
 
@@ -502,9 +482,6 @@ int fsl_destroy(fsl_ctx *h)
     if (c.faces_alloc)
         for (int s = 0; s < 2; s++)
             for (int v = 0; v < 5; v++) { cudaFree(c.f.x[s][v]); cudaFree(c.f.y[s][v]); cudaFree(c.f.z[s][v]); }
-    if (c.dyn_alloc) {
-        cudaFree(c.dyn.vel); cudaFree(c.dyn.F); cudaFree(c.dyn.A); cudaFree(c.dyn.S);
-    }
     if (c.bf_alloc) {
         cudaFree(c.bf.x0); cudaFree(c.bf.xL); cudaFree(c.bf.y0);
         cudaFree(c.bf.yH); cudaFree(c.bf.z0); cudaFree(c.bf.zD);
@@ -513,7 +490,6 @@ int fsl_destroy(fsl_ctx *h)
     if (c.fp32_alloc) {
         cudaFree(c.bf32.x0); cudaFree(c.bf32.xL); cudaFree(c.bf32.y0);
         cudaFree(c.bf32.yH); cudaFree(c.bf32.z0); cudaFree(c.bf32.zD); cudaFree(c.mu32);
-        cudaFree(c.dyn32.vel); cudaFree(c.dyn32.F); cudaFree(c.dyn32.A); cudaFree(c.dyn32.S);
     }
     for (auto &r : c.recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     for (auto e : c.evpool) cudaEventDestroy(e);
@@ -880,8 +856,6 @@ int fsl_dynamic_smagorinsky(fsl_ctx *h)
     if (!h) return FSL_ERR_ARG;
     Ctx &c = h->c;
     if (c.stage_next != 0) return fail(c, FSL_ERR_ARG, "fsl_dynamic_smagorinsky: a step is in progress (fsl_step_stage)");
-    int rc = ensure_dyn(c);
-    if (rc) return rc;
     launch_dynsmag(c, c.U);
     CKL();
     return FSL_OK;
@@ -954,7 +928,7 @@ namespace fsl {
 int step_prelude32(Ctx &c)
 {
     int rc;
-    if ((rc = ensure_dyn(c)) || (rc = ensure_bf(c)) || (rc = ensure_fp32(c))) return rc;
+    if ((rc = ensure_bf(c)) || (rc = ensure_fp32(c))) return rc;
     if (c.co_valid) launch_courant_apply(c);
     else launch_courant(c);
     c.step++;
@@ -1002,7 +976,6 @@ int fsl_step_phased(fsl_ctx *h, int nsteps)
         draw(c);
         for (int s = 1; s <= c.p.nStages; s++) {
             if ((rc = ensure_faces(c))) return rc;
-            if ((rc = ensure_dyn(c))) return rc;
             double *cur = cur_ptr(c);
             launch_ghost(c, cur);
             launch_recon(c, cur);
@@ -1041,7 +1014,6 @@ int fsl_step(fsl_ctx *h, int nsteps)
     }
     int rc;
     if ((rc = slab_check(c, nsteps))) return rc;
-    if ((rc = ensure_dyn(c))) return rc;
     if ((rc = ensure_bf(c))) return rc;
     if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step: the current-stage buffer is not U^n");
     if (c.p.precision == FSL_PREC_FP32) {
@@ -1115,7 +1087,6 @@ int fsl_step_stage(fsl_ctx *h)
     int rc;
     if (c.stage_next == 0) {
         if ((rc = slab_check(c, 1))) return rc;
-        if ((rc = ensure_dyn(c))) return rc;
         if ((rc = ensure_bf(c))) return rc;
         if (fp32 && (rc = ensure_fp32(c))) return rc;
         if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step_stage: the current-stage buffer is not U^n");

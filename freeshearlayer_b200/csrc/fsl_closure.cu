@@ -312,7 +312,7 @@ int fsl_closure_compare(fsl_ctx *h, float *cs2_mlp, float *cs2_dyn, fsl_closure_
     if (!c.cl_alloc || !c.cl_weights) return FSL_ERR_ARG;
     int rc = 0;
     launch_ghost(c, c.U);
-    if ((rc = ensure_dyn_scratch(c))) return rc;
+    if ((rc = ensure_sgs(c))) return rc;
     if ((rc = judge_now(c))) return rc;
     if (errs) fsl_closure_get_stats(h, errs);
     const Grid &g = c.g;
@@ -380,7 +380,7 @@ int fsl_trainer_harvest(fsl_trainer *t, fsl_ctx *h, int stride)
     int rc = ensure_closure(c);
     if (rc) return rc;
     if (c.cls.DD == 0.f) return FSL_ERR_ARG; // fsl_closure_set_scales first
-    if ((rc = ensure_dyn_scratch(c))) return rc;
+    if ((rc = ensure_sgs(c))) return rc;
     launch_ghost(c, c.U);
     launch_dynsmag(c, c.U, c.cd32);
     if (c.g.L < 5 || c.g.H < 5 || c.g.D < 5) return FSL_ERR_ARG;

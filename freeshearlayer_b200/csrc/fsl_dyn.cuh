@@ -1,5 +1,5 @@
-// fsl_dyn.cuh -- the dynamic Smagorinsky procedure (src/turbulence.c:17-507)
-// as seven passes, templated on the arithmetic type T: T = double in
+// fsl_dyn.cuh -- the dynamic Smagorinsky procedure (src/turbulence.c:17-507),
+// as one marching kernel and as separate passes, templated on the arithmetic type T: T = double in
 // fsl_phase.cu (the plain method, compiled with --fmad=false, bit-identical to
 // the reference) and T = float in fsl_dyn32.cu (the FP32-bulk path's
 // filtering and coefficient).  The conserved state U stays FP64 in both.
@@ -199,309 +199,273 @@ __global__ void k_dyn_final(Grid g, Consts kc, const double *__restrict__ rho, c
 
 
 // ---------------------------------------------------------------------------
-// Fused evaluation: the same arithmetic in three streaming kernels.
+// Fused evaluation: the same arithmetic in one kernel that marches along x.
 //
-// k_dyn_filter9 marches along x over a (TJ rows x 32 k) tile of output
-// positions: per plane it stages the velocities (halo 1 in y and z) in shared
-// memory, forms the y pass of u, v, w and their six products, the z pass per
-// own position, and the x pass from the last three z-pass planes it keeps in
-// registers -- each sum as t = 0; t += a h; t += b h; t += c h, on the
-// reference's write regions (pass 1: i in [0,L], j in [1,H], k in [0,D];
-// pass 2: k in [1,D]; pass 3: i in [1,L]; plane 0 keeps the y-pass value,
-// src/turbulence.c:44-95).  Positions outside those regions are never
-// written and stay zero, so the output equals the seven-pass result
-// everywhere.  k_dyn_strain forms A = |S| S and |S| of the interior
-// (src/turbulence.c:273-311).  k_dyn_filterA_final filters A the same way
-// (A is zero outside the interior, where the zero bands and a plain filter
-// agree) and, per interior cell, forms the Leonard stress, |S^| S^ from the
-// filtered velocities, M, the clipped coefficient and mu_SGS
-// (src/turbulence.c:250-445) without storing L or B.
+// A block owns DYN_J rows x DYN_K columns of output cells; its warps are the
+// rows with a one-row halo and its lanes the columns with a two-column halo, so
+// every neighbour along z is a lane and every neighbour along y a row of shared
+// memory.  Per plane p of velocities it forms
+//   - the box filter of u, v, w and their six products: the y pass from the rows'
+//     values h q in shared memory, the z pass by shuffles of h t1, the x pass as
+//     two running sums -- each sum as 0 + a h + b h + c h, each product by h
+//     formed once (the reference forms it three times; the same value);
+//   - the filtered velocities and the Leonard stress of plane p-1, and the
+//     strain rate and A = |S| S of plane p-1, filtered the same way;
+//   - from these |S^| S^, M, the clipped coefficient and mu_SGS of plane p-2
+//     (src/turbulence.c:250-445).
+// The filter's write regions are the reference's (pass 1: i in [0,L], j in
+// [1,H], k in [0,D]; pass 2: k in [1,D]; pass 3: i in [1,L]; plane 0 keeps the
+// y-pass value, src/turbulence.c:44-95), zero elsewhere; A is zero outside the
+// interior.
+//
+// Four streaming kernels (velocities, filter, strain, filter of A) with 19
+// scratch fields went before: 376 B of traffic a cell and a march of 32 planes
+// per block whatever the grid.  This one reads the state once per block, keeps
+// everything else on chip (no scratch fields), and cuts the march so that the
+// blocks fill the SMs.  It is bound by the latency of shared memory, shuffles and
+// dependent arithmetic at 16 warps an SM (issue slots 42 % busy in FP64, 60 %
+// in FP32).  Measured: FP64 512x256x256 4.21 -> 3.15 ms, 64x32x32 177 -> 35 us;
+// FP32 203x97x75 195 -> 78 us.
 // ---------------------------------------------------------------------------
-template <typename T> struct Scratch3 {
-    T *vel; // 3 fields
-    T *F;   // 9 fields, zero outside the filter's write regions (never written there)
-    T *A;   // 6 fields, zero on the ghost layer (never written there)
-    T *S;   // |S| of the interior
+constexpr int DYN_W = 16, DYN_J = DYN_W - 2, DYN_K = 28; // warps, output rows, output columns
+
+template <typename T> struct DynSmem {
+    double raw[4][DYN_W * 32 + 64];  // rho, rho u, rho v, rho w of the next plane, in flight (own slots)
+    T Q[DYN_W + 2][32][9];           // h times u v w uu uv uw vv vw ww of plane p
+    T V[2][DYN_W + 2][32][3];        // velocities of planes p, p-1
+    T F[2][DYN_W][32][3];            // filtered velocities of planes p-1, p-2
+    T A[DYN_W][32][6];               // h A of plane p-1
+    // running x sums of the nine filters: FP64 in shared memory (own slots), as
+    // registers they would spill at 128 a thread; FP32 in registers
+    static constexpr bool XS = sizeof(T) == 8;
+    T X[XS ? 18 : 1][DYN_W * 32];
 };
 
-template <typename T, int TJ>
-__global__ void __launch_bounds__(32 * TJ) k_dyn_filter9(Grid g, int seg, const T *__restrict__ vel, T *__restrict__ F)
+template <typename T> __device__ __forceinline__ T sh_up(T v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+template <typename T> __device__ __forceinline__ T sh_dn(T v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+
+// |S| and S (11 12 13 22 23 33) from the differences d[a][x] of velocity
+// component a along axis x (src/turbulence.c:273-311, :316-366)
+template <typename T> __device__ __forceinline__ T strain_of(const T (*d)[3], T *S)
 {
-    __shared__ T vq[TJ + 2][34][3];
-    __shared__ T t1[TJ][34][9];
+    S[0] = d[0][0];
+    S[1] = T(0.5) * (d[0][1] + d[1][0]);
+    S[2] = T(0.5) * (d[0][2] + d[2][0]);
+    S[3] = d[1][1];
+    S[4] = T(0.5) * (d[1][2] + d[2][1]);
+    S[5] = d[2][2];
+    const T S21 = S[1], S31 = S[2], S32 = S[4];
+    return sqrt(2 * (S[0] * S[0] + S[1] * S[1] + S[2] * S[2] + S21 * S21 + S[3] * S[3] + S[4] * S[4] + S31 * S31 +
+                     S32 * S32 + S[5] * S[5]));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DYN_W * 32, 1)
+    k_dyn_march(Grid g, Consts kc, int seg, const double *__restrict__ U, T *__restrict__ mu, float *__restrict__ cd)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    DynSmem<T> &s = *reinterpret_cast<DynSmem<T> *>(smraw);
     const int L = g.L, H = g.H, D = g.D;
-    const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l, nt = 32 * TJ;
-    const int k0 = blockIdx.x * 32, j0 = 1 + blockIdx.y * TJ;
-    const int j = j0 + r, k = k0 + l;
-    const int i0 = blockIdx.z * seg, i1 = min(L, i0 + seg - 1);
+    const int t = threadIdx.x, l = t & 31, r = t >> 5;
+    const int j = (int)blockIdx.y * DYN_J + r, k = (int)blockIdx.x * DYN_K + l - 1; // row 1, lane 2: the first output cell
+    const int i0 = 1 + (int)blockIdx.z * seg, i1 = min(L, i0 + seg - 1);
     const long long fs = g.fstride;
-    const bool own = j <= H && k <= D;
-    T p2[9], p1[9], cur[9];
+    const T h = T(H3), r2x = T(kc.r2dx), r2y = T(kc.r2dy), r2z = T(kc.r2dz);
+    // the rows below warp 0's and above the last warp's: an extra cell of those warps
+    const bool edge = r == 0 || r == DYN_W - 1;
+    const int je = r == 0 ? j - 1 : j + 1;
+    const bool kin = k >= 0 && k <= D + 1;
+    const bool in = kin && j <= H + 1, ein = edge && kin && je >= 0 && je <= H + 1;
+    const long long c0 = in ? g.idx(0, j, k) : 0, ce = ein ? g.idx(0, je, k) : 0;
+    const bool y1 = j >= 1 && j <= H && k >= 0 && k <= D; // pass 1 writes here
+    const bool z1 = y1 && k >= 1;                         // pass 2, and the interior
+    const bool own = z1 && r >= 1 && r <= DYN_J && l >= 2 && l <= DYN_K + 1;
+
+    auto fetch = [&](int p) {
+        if (p >= 0 && p <= L + 1) {
 #pragma unroll
-    for (int m = 0; m < 9; m++) p2[m] = p1[m] = cur[m] = T(0.);
-    const int ib = max(i0 - 1, 0), ie = min(i1 + 1, L + 1);
-    // the staged region (TJ+2) x 34 of a plane, at most two positions per
-    // thread; plane ip+1 is loaded into registers while plane ip is filtered
-    constexpr int NP = ((TJ + 2) * 34 + 32 * TJ - 1) / (32 * TJ);
-    T pre[NP][3];
-    auto issue = [&](int ip) {
+            for (int w = 0; w < 2; w++) {
+                if (w ? !ein : !in) continue;
+                const long long c = FSL_CELL((w ? ce : c0) + p * g.pi, fs);
+                const int slot = w ? DYN_W * 32 + (r ? 32 : 0) + l : t;
 #pragma unroll
-        for (int s = 0; s < NP; s++) {
-            const int e = tid + s * nt;
-            const int rr = e / 34, cc = e % 34, jj = j0 - 1 + rr, kk = k0 - 1 + cc;
-            pre[s][0] = pre[s][1] = pre[s][2] = T(0.);
-            if (e < (TJ + 2) * 34 && ip <= L && jj <= H + 1 && kk >= 0 && kk <= D + 1) {
-                const long long q = FSL_CELL(g.idx(ip, jj, kk), fs);
-                pre[s][0] = vel[q]; pre[s][1] = vel[fs + q]; pre[s][2] = vel[2 * fs + q];
+                for (int q = 0; q < 4; q++)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(&s.raw[q][slot])),
+                                 "l"(U + q * fs + c)
+                                 : "memory");
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    issue(ib);
-    for (int ip = ib; ip <= ie; ip++) {
-        if (ip <= L) {
+
+    T v1[3] = {}, v2[3] = {};       // own velocities of planes p-1, p-2
+    T f1[3] = {}, f2[3] = {};       // own filtered velocities of planes p-2, p-3
+    T Lst[6] = {};                  // Leonard stress of plane p-2
+    T a1[6] = {}, a2[6] = {};       // running x sums of the filter of A
+    T S1 = T(0.);                   // |S| of plane p-2
+    T t0[3] = {};                   // the y pass of plane 0
+    double r1 = 0., r2 = 0.;        // density of planes p-1, p-2
+    T x1[9] = {}, x2[9] = {};       // running x sums of the nine filters (FP32)
+    if constexpr (DynSmem<T>::XS) {
 #pragma unroll
-            for (int s = 0; s < NP; s++) {
-                const int e = tid + s * nt;
-                if (e < (TJ + 2) * 34) {
-                    const int rr = e / 34, cc = e % 34;
-                    vq[rr][cc][0] = pre[s][0]; vq[rr][cc][1] = pre[s][1]; vq[rr][cc][2] = pre[s][2];
-                }
+        for (int m = 0; m < 18; m++) s.X[m][t] = T(0.);
+    }
+    const int pb = max(i0 - 2, 0);
+    fetch(pb);
+    for (int p = pb; p <= i1 + 2; p++) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory"); // own copies only: no barrier
+        // ---- velocities and h q of plane p
+        T v0[3] = {};
+        double rho = 0.;
+        const bool pin = p <= L + 1;
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            if (w && !edge) continue;
+            T v[3] = {};
+            if (pin && (w ? ein : in)) {
+                const int slot = w ? DYN_W * 32 + (r ? 32 : 0) + l : t;
+                const double rw = s.raw[0][slot];
+                const T rr = T(1.) / T(rw);
+                v[0] = T(s.raw[1][slot]) * rr;
+                v[1] = T(s.raw[2][slot]) * rr;
+                v[2] = T(s.raw[3][slot]) * rr;
+                if (!w) rho = rw;
             }
-            issue(ip + 1);
-            __syncthreads();
-            // pass 1 (y) of the nine fields at rows j0.., columns k0-1 .. k0+32
-            for (int e = tid; e < TJ * 34; e += nt) {
-                const int rr = e / 34, cc = e % 34, jj = j0 + rr, kk = k0 - 1 + cc;
-                T o[9];
-                if (jj <= H && kk >= 0 && kk <= D) {
-                    T q[3][9];
-#pragma unroll
-                    for (int w = 0; w < 3; w++) {
-                        const T uu = vq[rr + w][cc][0], vv = vq[rr + w][cc][1], ww = vq[rr + w][cc][2];
-                        q[w][0] = uu; q[w][1] = vv; q[w][2] = ww;
-                        q[w][3] = uu * uu; q[w][4] = uu * vv; q[w][5] = uu * ww;
-                        q[w][6] = vv * vv; q[w][7] = vv * ww; q[w][8] = ww * ww;
-                    }
-#pragma unroll
-                    for (int m = 0; m < 9; m++) {
-                        T t = 0.;
-                        t += q[0][m] * T(H3); t += q[1][m] * T(H3); t += q[2][m] * T(H3);
-                        o[m] = t;
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < 9; m++) o[m] = T(0.);
-                }
-#pragma unroll
-                for (int m = 0; m < 9; m++) t1[rr][cc][m] = o[m];
-            }
-            __syncthreads();
-            // pass 2 (z) at the own position
-            if (own && k >= 1) {
-#pragma unroll
-                for (int m = 0; m < 9; m++) {
-                    T t = 0.;
-                    t += t1[r][l][m] * T(H3); t += t1[r][l + 1][m] * T(H3); t += t1[r][l + 2][m] * T(H3);
-                    cur[m] = t;
-                }
-            } else {
-#pragma unroll
-                for (int m = 0; m < 9; m++) cur[m] = T(0.);
-            }
-            // plane 0 keeps its pass-1 value
-            if (ip == 0 && own) {
-                const long long c = FSL_CELL(g.idx(0, j, k), fs);
-#pragma unroll
-                for (int m = 0; m < 9; m++) F[m * fs + c] = t1[r][l + 1][m];
-            }
-            __syncthreads(); // the next plane overwrites vq and t1
-        } else {
-#pragma unroll
-            for (int m = 0; m < 9; m++) cur[m] = T(0.); // plane L+1: pass 2 writes nothing there
+            const int row = w ? (r ? DYN_W + 1 : 0) : r + 1;
+            T *q = s.Q[row][l], *o = s.V[p & 1][row][l];
+            o[0] = v[0]; o[1] = v[1]; o[2] = v[2];
+            q[0] = v[0] * h; q[1] = v[1] * h; q[2] = v[2] * h;
+            q[3] = v[0] * v[0] * h; q[4] = v[0] * v[1] * h; q[5] = v[0] * v[2] * h;
+            q[6] = v[1] * v[1] * h; q[7] = v[1] * v[2] * h; q[8] = v[2] * v[2] * h;
+            if (!w) { v0[0] = v[0]; v0[1] = v[1]; v0[2] = v[2]; }
         }
-        // pass 3 (x) of plane ip-1
-        const int io = ip - 1;
-        if (io >= max(i0, 1) && io <= i1 && own && k >= 1) {
-            const long long c = FSL_CELL(g.idx(io, j, k), fs);
+        __syncthreads();
+        if (p < i1 + 2) fetch(p + 1);
+        // ---- the nine filters: F of plane p-1
+        T fn[3], Ln[6];
+        {
+            const bool yp = y1 && p <= L, zp = z1 && p <= L;
+            T F[9];
 #pragma unroll
             for (int m = 0; m < 9; m++) {
-                T t = 0.;
-                t += p2[m] * T(H3); t += p1[m] * T(H3); t += cur[m] * T(H3);
-                F[m * fs + c] = t;
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < 9; m++) {
-            p2[m] = p1[m];
-            p1[m] = cur[m];
-        }
-    }
-}
-
-// A_ij = |S| S_ij and |S| of the interior from the velocities (pass 0 of
-// k_dyn_mid: the same expressions).
-template <typename T>
-__global__ void k_dyn_strain(Grid g, Consts kc, const T *__restrict__ vel, T *__restrict__ A, T *__restrict__ Smag)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int i = blockIdx.z + 1;
-    if (k > g.D || j > g.H) return;
-    const long long fs = g.fstride, c = g.idx(i, j, k);
-    if (!FSL_SPAN(c, -g.pi, g.pi, fs)) return;
-    const long long dI = g.pi, dJ = g.pk;
-    const T *uu = vel, *vv = vel + fs, *ww = vel + 2 * fs;
-    const T du_dx = (uu[c + dI] - uu[c - dI]) * T(kc.r2dx);
-    const T du_dy = (uu[c + dJ] - uu[c - dJ]) * T(kc.r2dy);
-    const T du_dz = (uu[c + 1] - uu[c - 1]) * T(kc.r2dz);
-    const T dv_dx = (vv[c + dI] - vv[c - dI]) * T(kc.r2dx);
-    const T dv_dy = (vv[c + dJ] - vv[c - dJ]) * T(kc.r2dy);
-    const T dv_dz = (vv[c + 1] - vv[c - 1]) * T(kc.r2dz);
-    const T dw_dx = (ww[c + dI] - ww[c - dI]) * T(kc.r2dx);
-    const T dw_dy = (ww[c + dJ] - ww[c - dJ]) * T(kc.r2dy);
-    const T dw_dz = (ww[c + 1] - ww[c - 1]) * T(kc.r2dz);
-    const T S11 = du_dx, S12 = T(0.5) * (du_dy + dv_dx), S13 = T(0.5) * (du_dz + dw_dx);
-    const T S21 = S12, S22 = dv_dy, S23 = T(0.5) * (dv_dz + dw_dy);
-    const T S31 = S13, S32 = S23, S33 = dw_dz;
-    const T S = sqrt(2 * (S11 * S11 + S12 * S12 + S13 * S13 + S21 * S21 + S22 * S22 + S23 * S23 + S31 * S31 +
-                          S32 * S32 + S33 * S33));
-    A[c] = S * S11; A[fs + c] = S * S12; A[2 * fs + c] = S * S13;
-    A[3 * fs + c] = S * S22; A[4 * fs + c] = S * S23; A[5 * fs + c] = S * S33;
-    Smag[c] = S;
-}
-
-template <typename T, int TJ>
-__global__ void __launch_bounds__(32 * TJ)
-    k_dyn_filterA_final(Grid g, Consts kc, int seg, const double *__restrict__ rho, const T *__restrict__ F,
-                        const T *__restrict__ A, const T *__restrict__ Smag, T *__restrict__ mu,
-                        float *__restrict__ cd)
-{
-    __shared__ T qa[TJ + 2][34][6];
-    __shared__ T t1[TJ][34][6];
-    const int L = g.L, H = g.H, D = g.D;
-    const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l, nt = 32 * TJ;
-    const int k0 = 1 + blockIdx.x * 32, j0 = 1 + blockIdx.y * TJ;
-    const int j = j0 + r, k = k0 + l;
-    const int i0 = 1 + blockIdx.z * seg, i1 = min(L, i0 + seg - 1);
-    const long long fs = g.fstride;
-    const bool own = j <= H && k <= D;
-    T p2[6], p1[6], cur[6];
-#pragma unroll
-    for (int m = 0; m < 6; m++) p2[m] = p1[m] = cur[m] = T(0.);
-    constexpr int NP = ((TJ + 2) * 34 + 32 * TJ - 1) / (32 * TJ);
-    T pre[NP][6];
-    auto issue = [&](int ip) {
-#pragma unroll
-        for (int s = 0; s < NP; s++) {
-            const int e = tid + s * nt;
-            const int rr = e / 34, cc = e % 34, jj = j0 - 1 + rr, kk = k0 - 1 + cc;
-#pragma unroll
-            for (int m = 0; m < 6; m++) pre[s][m] = T(0.);
-            if (e < (TJ + 2) * 34 && ip >= 1 && ip <= L && jj <= H + 1 && kk <= D + 1) {
-                const long long q = FSL_CELL(g.idx(ip, jj, kk), fs);
-#pragma unroll
-                for (int m = 0; m < 6; m++) pre[s][m] = A[m * fs + q];
-            }
-        }
-    };
-    issue(i0 - 1);
-    for (int ip = i0 - 1; ip <= i1 + 1; ip++) {
-        if (ip >= 1 && ip <= L) { // A is zero on the planes 0 and L+1
-#pragma unroll
-            for (int s = 0; s < NP; s++) {
-                const int e = tid + s * nt;
-                if (e < (TJ + 2) * 34) {
-                    const int rr = e / 34, cc = e % 34;
-#pragma unroll
-                    for (int m = 0; m < 6; m++) qa[rr][cc][m] = pre[s][m];
+                T t1 = T(0.) + s.Q[r][l][m];
+                t1 += s.Q[r + 1][l][m];
+                t1 += s.Q[r + 2][l][m];
+                if (!yp) t1 = T(0.);
+                const T th = t1 * h;
+                T t2 = T(0.) + sh_up(th);
+                t2 += th;
+                t2 += sh_dn(th);
+                if (!zp) t2 = T(0.);
+                const T x = t2 * h;
+                if constexpr (DynSmem<T>::XS) {
+                    F[m] = s.X[9 + m][t] + x;
+                    s.X[9 + m][t] = s.X[m][t] + x;
+                    s.X[m][t] = T(0.) + x;
+                } else {
+                    F[m] = x2[m] + x;
+                    x2[m] = x1[m] + x;
+                    x1[m] = T(0.) + x;
+                }
+                if (m < 3) {
+                    if (p == 1) F[m] = t0[m]; // plane 0 keeps the y pass
+                    if (p == 0) t0[m] = t1;
                 }
             }
-            issue(ip + 1);
-            __syncthreads();
-            for (int e = tid; e < TJ * 34; e += nt) {
-                const int rr = e / 34, cc = e % 34, jj = j0 + rr, kk = k0 - 1 + cc;
-                const bool in = jj <= H && kk <= D;
+            const bool none = p > L + 1 || p == 0; // nothing is written on plane L+1 (and none precedes plane 0)
 #pragma unroll
-                for (int m = 0; m < 6; m++) {
-                    T t = 0.;
-                    if (in) {
-                        t += qa[rr][cc][m] * T(H3); t += qa[rr + 1][cc][m] * T(H3); t += qa[rr + 2][cc][m] * T(H3);
-                    }
-                    t1[rr][cc][m] = t;
-                }
+            for (int m = 0; m < 3; m++) {
+                fn[m] = none ? T(0.) : F[m];
+                s.F[(p + 1) & 1][r][l][m] = fn[m];
             }
-            __syncthreads();
-            if (own) {
-#pragma unroll
-                for (int m = 0; m < 6; m++) {
-                    T t = 0.;
-                    t += t1[r][l][m] * T(H3); t += t1[r][l + 1][m] * T(H3); t += t1[r][l + 2][m] * T(H3);
-                    cur[m] = t;
-                }
-            }
-            __syncthreads();
-        } else {
-#pragma unroll
-            for (int m = 0; m < 6; m++) cur[m] = T(0.);
-            if (ip == 0) issue(1); // the march starts on plane 0 (i0 = 1)
+            Ln[0] = F[3] - F[0] * F[0]; Ln[1] = F[4] - F[0] * F[1]; Ln[2] = F[5] - F[0] * F[2];
+            Ln[3] = F[6] - F[1] * F[1]; Ln[4] = F[7] - F[1] * F[2]; Ln[5] = F[8] - F[2] * F[2];
         }
-        const int io = ip - 1;
-        if (io >= i0 && io <= i1 && own) {
+        // ---- strain rate of plane p-1: A and |S|
+        T S0 = T(0.);
+        {
+            T d[3][3], A[6];
+            const T(*V)[32][3] = s.V[(p + 1) & 1];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                d[a][0] = (v0[a] - v2[a]) * r2x;
+                d[a][1] = (V[r + 2][l][a] - V[r][l][a]) * r2y;
+                const T up = sh_dn(v1[a]), dn = sh_up(v1[a]);
+                d[a][2] = (up - dn) * r2z;
+            }
+            const bool ap = z1 && p >= 2 && p <= L + 1;
+            S0 = strain_of(d, A);
+#pragma unroll
+            for (int m = 0; m < 6; m++) s.A[r][l][m] = ap ? S0 * A[m] * h : T(0.);
+        }
+        __syncthreads();
+        // ---- the filter of A, and plane p-2
+        const bool mid = r >= 1 && r <= DYN_J;
+        if (mid) {
             T Ah[6];
 #pragma unroll
             for (int m = 0; m < 6; m++) {
-                T t = 0.;
-                t += p2[m] * T(H3); t += p1[m] * T(H3); t += cur[m] * T(H3);
-                Ah[m] = t;
+                T t1 = T(0.) + s.A[r - 1][l][m];
+                t1 += s.A[r][l][m];
+                t1 += s.A[r + 1][l][m];
+                if (!y1) t1 = T(0.);
+                const T th = t1 * h;
+                T t2 = T(0.) + sh_up(th);
+                t2 += th;
+                t2 += sh_dn(th);
+                const T x = (p >= 2 && p <= L + 1) ? t2 * h : T(0.);
+                Ah[m] = a2[m] + x;
+                a2[m] = a1[m] + x;
+                a1[m] = T(0.) + x;
             }
-            const long long c = FSL_CELL(g.idx(io, j, k), fs);
-            (void)FSL_SPAN(c, -g.pi, g.pi, fs); // its strain stencil (the block barriers forbid a skip)
-            // Leonard stress (src/turbulence.c:250-270)
-            const T f0 = F[c], f1 = F[fs + c], f2 = F[2 * fs + c];
-            T L11 = F[3 * fs + c] - f0 * f0, L12 = F[4 * fs + c] - f0 * f1, L13 = F[5 * fs + c] - f0 * f2;
-            T L22 = F[6 * fs + c] - f1 * f1, L23 = F[7 * fs + c] - f1 * f2, L33 = F[8 * fs + c] - f2 * f2;
-            // |S^| S^ from the filtered velocities (pass 1 of k_dyn_mid)
-            const long long dI = g.pi, dJ = g.pk;
-            const T *uu = F, *vv = F + fs, *ww = F + 2 * fs;
-            const T du_dx = (uu[c + dI] - uu[c - dI]) * T(kc.r2dx);
-            const T du_dy = (uu[c + dJ] - uu[c - dJ]) * T(kc.r2dy);
-            const T du_dz = (uu[c + 1] - uu[c - 1]) * T(kc.r2dz);
-            const T dv_dx = (vv[c + dI] - vv[c - dI]) * T(kc.r2dx);
-            const T dv_dy = (vv[c + dJ] - vv[c - dJ]) * T(kc.r2dy);
-            const T dv_dz = (vv[c + 1] - vv[c - 1]) * T(kc.r2dz);
-            const T dw_dx = (ww[c + dI] - ww[c - dI]) * T(kc.r2dx);
-            const T dw_dy = (ww[c + dJ] - ww[c - dJ]) * T(kc.r2dy);
-            const T dw_dz = (ww[c + 1] - ww[c - 1]) * T(kc.r2dz);
-            const T S11 = du_dx, S12 = T(0.5) * (du_dy + dv_dx), S13 = T(0.5) * (du_dz + dw_dx);
-            const T S21 = S12, S22 = dv_dy, S23 = T(0.5) * (dv_dz + dw_dy);
-            const T S31 = S13, S32 = S23, S33 = dw_dz;
-            const T Sh = sqrt(2 * (S11 * S11 + S12 * S12 + S13 * S13 + S21 * S21 + S22 * S22 + S23 * S23 +
-                                   S31 * S31 + S32 * S32 + S33 * S33));
-            // M_ij, coefficient, mu_SGS (src/turbulence.c:398-445; k_dyn_final)
-            const T DD = T(kc.DD);
-            const T M11 = DD * (4 * (Sh * S11) - Ah[0]);
-            const T M12 = DD * (4 * (Sh * S12) - Ah[1]);
-            const T M13 = DD * (4 * (Sh * S13) - Ah[2]);
-            const T M22 = DD * (4 * (Sh * S22) - Ah[3]);
-            const T M23 = DD * (4 * (Sh * S23) - Ah[4]);
-            const T M33 = DD * (4 * (Sh * S33) - Ah[5]);
-            const T tr = T(-(1.0 / 3.0)) * (L11 + L22 + L33);
-            L11 += tr; L22 += tr; L33 += tr;
-            const T LLMM = (L11 * M11 + L12 * M12 + L13 * M13 + L12 * M12 + L22 * M22 + L23 * M23 + L13 * M13 +
-                            L23 * M23 + L33 * M33);
-            const T MMMM = (M11 * M11 + M12 * M12 + M13 * M13 + M12 * M12 + M22 * M22 + M23 * M23 + M13 * M13 +
-                            M23 * M23 + M33 * M33);
-            T Cd = T(-0.5) * (LLMM / (MMMM + T(1e-30)));
-            if (Cd > T(0.15)) Cd = T(0.15);
-            else if (Cd < T(0.0)) Cd = T(0.0);
-            mu[c] = T(rho[c]) * Cd * DD * Smag[c];
-            if (cd) cd[c] = (float)Cd;
+            T d[3][3], Sh_[6];
+            const T(*F)[32][3] = s.F[p & 1];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                d[a][0] = (fn[a] - f2[a]) * r2x;
+                d[a][1] = (F[r + 1][l][a] - F[r - 1][l][a]) * r2y;
+                const T up = sh_dn(f1[a]), dn = sh_up(f1[a]);
+                d[a][2] = (up - dn) * r2z;
+            }
+            const int io = p - 2;
+            if (own && io >= i0) {
+                const T Sh = strain_of(d, Sh_);
+                const T DD = T(kc.DD);
+                const T M11 = DD * (4 * (Sh * Sh_[0]) - Ah[0]);
+                const T M12 = DD * (4 * (Sh * Sh_[1]) - Ah[1]);
+                const T M13 = DD * (4 * (Sh * Sh_[2]) - Ah[2]);
+                const T M22 = DD * (4 * (Sh * Sh_[3]) - Ah[3]);
+                const T M23 = DD * (4 * (Sh * Sh_[4]) - Ah[4]);
+                const T M33 = DD * (4 * (Sh * Sh_[5]) - Ah[5]);
+                T L11 = Lst[0], L22 = Lst[3], L33 = Lst[5];
+                const T L12 = Lst[1], L13 = Lst[2], L23 = Lst[4];
+                const T tr = T(-(1.0 / 3.0)) * (L11 + L22 + L33);
+                L11 += tr; L22 += tr; L33 += tr;
+                const T LLMM = (L11 * M11 + L12 * M12 + L13 * M13 + L12 * M12 + L22 * M22 + L23 * M23 + L13 * M13 +
+                                L23 * M23 + L33 * M33);
+                const T MMMM = (M11 * M11 + M12 * M12 + M13 * M13 + M12 * M12 + M22 * M22 + M23 * M23 + M13 * M13 +
+                                M23 * M23 + M33 * M33);
+                T Cd = T(-0.5) * (LLMM / (MMMM + T(1e-30)));
+                if (Cd > T(0.15)) Cd = T(0.15);
+                else if (Cd < T(0.0)) Cd = T(0.0);
+                const long long c = FSL_CELL(c0 + io * g.pi, fs);
+                mu[c] = T(r2) * Cd * DD * S1;
+                if (cd) cd[c] = (float)Cd;
+            }
+        }
+        S1 = S0;
+        r2 = r1;
+        r1 = rho;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            v2[a] = v1[a];
+            v1[a] = v0[a];
+            f2[a] = f1[a];
+            f1[a] = fn[a];
         }
 #pragma unroll
-        for (int m = 0; m < 6; m++) {
-            p2[m] = p1[m];
-            p1[m] = cur[m];
-        }
+        for (int m = 0; m < 6; m++) Lst[m] = Ln[m];
     }
 }
 
@@ -537,22 +501,30 @@ void sequence(const Grid &g, const Consts &k, const Scratch<T> &s, const double 
     k_dyn_final<T><<<cells_grid3(b, g.L, g.H, g.D), b, 0, st>>>(g, k, U, s.Lst, s.B, s.t1, s.S, mu, cd);
 }
 
-// The fused evaluation: velocities, the nine-field filter, A and |S|, the
-// filter of A with the coefficient and mu_SGS -- four launches.
+// The fused evaluation: one launch.  The march is cut so that the blocks fill
+// the SMs in whole waves: a segment of n planes costs n + 4 (the planes its
+// filters reach), and the number of waves times that is least.
 template <typename T>
-void sequence_fused(const Grid &g, const Consts &k, const Scratch3<T> &s, const double *U, T *mu, float *cd,
-                    cudaStream_t st)
+int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int sms, cudaStream_t st)
 {
-    constexpr int TJ = 8, SEG = 32;
-    const long long ncell = (long long)(g.L + 2) * g.pi;
-    k_dyn_vel<T><<<(unsigned)std::min<long long>((ncell + 255) / 256, 148LL * 16), 256, 0, st>>>(g, U, s.vel);
-    const dim3 bt(32, TJ, 1);
-    const dim3 g9((unsigned)((g.D + 1 + 31) / 32), (unsigned)((g.H + TJ - 1) / TJ), (unsigned)((g.L + 1 + SEG - 1) / SEG));
-    k_dyn_filter9<T, TJ><<<g9, bt, 0, st>>>(g, SEG, s.vel, s.F);
-    const dim3 b(32, 4, 1);
-    k_dyn_strain<T><<<cells_grid3(b, g.L, g.H, g.D), b, 0, st>>>(g, k, s.vel, s.A, s.S);
-    const dim3 g6((unsigned)((g.D + 31) / 32), (unsigned)((g.H + TJ - 1) / TJ), (unsigned)((g.L + SEG - 1) / SEG));
-    k_dyn_filterA_final<T, TJ><<<g6, bt, 0, st>>>(g, k, SEG, U, s.F, s.A, s.S, mu, cd);
+    static std::atomic<uint64_t> attr{0};
+    if (!smem_limit_once((const void *)k_dyn_march<T>, sizeof(DynSmem<T>), attr)) return -1;
+    const unsigned nk = (unsigned)((g.D + DYN_K - 1) / DYN_K), nj = (unsigned)((g.H + DYN_J - 1) / DYN_J);
+    const long long tiles = (long long)nk * nj;
+    int seg = 1;
+    long long best = -1;
+    for (int n = 1; n <= g.L; n++) {
+        const long long segs = (g.L + n - 1) / n;
+        if (n > 1 && segs == (g.L + n - 2) / (n - 1)) continue; // the same number of blocks with longer segments
+        const long long cost = (tiles * segs + sms - 1) / sms * (n + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            seg = n;
+        }
+    }
+    k_dyn_march<T><<<dim3(nk, nj, (unsigned)((g.L + seg - 1) / seg)), DYN_W * 32, sizeof(DynSmem<T>), st>>>(g, k, seg, U,
+                                                                                                          mu, cd);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 } // namespace dyn

@@ -74,17 +74,6 @@ struct BFaces32 {
     float *x0, *xL, *y0, *yH, *z0, *zD;
 };
 
-// Scratch of the dynamic Smagorinsky procedure (padded layout, FP64).
-// Scratch of the fused dynamic procedure (fsl_dyn.cuh, sequence_fused)
-template <typename T> struct DynFields {
-    T *vel; // 3 fields u, v, w
-    T *F;   // 9 fields: the filtered velocities and products; zero where no pass writes
-    T *A;   // 6 fields |S| S_ij, ghost layer kept zero
-    T *S;   // 1 field |S|
-};
-typedef DynFields<double> DynScratch;
-typedef DynFields<float> DynScratch32;
-
 struct Ctx {
     fsl_params p;
     Consts k;
@@ -97,9 +86,6 @@ struct Ctx {
     int cur = 0; // 0: U*_ = U, 1: U*_ = Up
     Faces f{};
     bool faces_alloc = false;
-    DynScratch dyn{};
-    DynScratch32 dyn32{}; // the FP32 path's own (a shared buffer would mix the two views' zero bands)
-    bool dyn_alloc = false;
     BFaces bf{};
     bool bf_alloc = false;
     // FP32-bulk path
@@ -181,7 +167,7 @@ struct Ctx {
 void prof_begin(Ctx &c, int cls);
 void prof_end(Ctx &c, int cls, int nkernels);
 
-int ensure_dyn_scratch(Ctx &c);  // SGS scratch of the dynamic procedure + the FP32 SGS field (fsl_api.cu)
+int ensure_sgs(Ctx &c);          // the FP32 path's SGS field (fsl_api.cu)
 int step_prelude32(Ctx &c);      // an FP32-bulk step up to its first stage (fsl_api.cu)
 int closure_step_sgs(Ctx &c);    // SGS of one step under FSL_SGS_LEARNED (fsl_closure.cu)
 int closure_ensure(Ctx &c);

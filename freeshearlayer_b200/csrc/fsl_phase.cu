@@ -677,11 +677,9 @@ void launch_evolution(Ctx &c, int nstages, int stage)
 
 void launch_dynsmag(Ctx &c, const double *U, float *cd)
 {
-    const DynScratch &s = c.dyn;
-    const dyn::Scratch3<double> sc{s.vel, s.F, s.A, s.S};
     prof_begin(c, FSL_K_SGS);
-    dyn::sequence_fused<double>(c.g, c.k, sc, U, c.mu, cd, c.stream);
-    prof_end(c, FSL_K_SGS, 4);
+    dyn::march<double>(c.g, c.k, U, c.mu, cd, c.sms, c.stream);
+    prof_end(c, FSL_K_SGS, 1);
 }
 
 void launch_courant(Ctx &c)
@@ -794,7 +792,7 @@ int noalloc_scratch(double **out)
 // The dynamic procedure's unfused nine-launch sequence (dyn::sequence: the
 // seven-pass filters and the coefficient, each field in its own scratch
 // array), on explicit buffers and stream.  The context path runs the fused
-// form (dyn::sequence_fused) on less scratch; both give the same bits.
+// form (dyn::march) without scratch; both give the same bits.
 void noalloc_dyn_sequence(const fsl::Grid &g, const fsl::Consts &k, const fsl::dyn::Scratch<double> &s,
                           const double *U, double *mu, cudaStream_t st)
 {
