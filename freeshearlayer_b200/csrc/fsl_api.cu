@@ -411,9 +411,10 @@ int fsl_init(const fsl_params *p, fsl_ctx **out)
     // x planes per fused-stage block: 48 measured fastest for the FP32 bulk
     // at 512x256x256 (1.6 % over 32); 32 for FP64
     c.stage_seg = (p->precision == FSL_PREC_FP32) ? 48 : 32;
-    // the FP32 bulk's reference-scheme stages run the full-lane persistent
-    // tile (rows 0); FP64 and PPM stages the ring tiles (rows 16)
-    c.stage_tje = (p->precision == FSL_PREC_FP32) ? 0 : 16;
+    // rows 0: the FP32 bulk's reference-scheme stages run the full-lane
+    // persistent tile, FP32 PPM stages the 16-row ring tile; FP64 stages pick
+    // their kernel and split by the grid (fsl_fused.cu)
+    c.stage_tje = 0;
     // derived constants, src/initialize.c:67-94
     c.k.rdx = 1. / p->deltaX; c.k.rdy = 1. / p->deltaY; c.k.rdz = 1. / p->deltaZ;
     c.k.r4dx = 1. / (4 * p->deltaX); c.k.r4dy = 1. / (4 * p->deltaY); c.k.r4dz = 1. / (4 * p->deltaZ);
@@ -888,13 +889,14 @@ int fsl_evolution(fsl_ctx *h, int stage)
     return FSL_OK;
 }
 
-// The FP32 bulk's full-lane stages on the temporal setup form the boundary
-// faces' outer states from the state itself and write the ghost cells of
-// their output: no boundary pass runs, and no ghost pass between stages.
-static bool wide_temporal(const Ctx &c)
+// On the temporal setup the FP32 bulk's full-lane stages and the FP64
+// direction-split stages form the boundary faces' outer states from the state
+// itself and write the ghost cells of their output (the FP64 ones not U^{n+1}'s):
+// no boundary pass runs, and no ghost pass between stages.
+static bool forms_boundaries(const Ctx &c)
 {
-    return c.p.precision == FSL_PREC_FP32 && c.p.recon == FSL_RECON_CHARMINMOD && c.stage_tje == 0 &&
-           c.p.setup == FSL_SETUP_TEMPORAL;
+    if (c.p.setup != FSL_SETUP_TEMPORAL || c.p.recon != FSL_RECON_CHARMINMOD || c.stage_tje != 0) return false;
+    return c.p.precision == FSL_PREC_FP32 || stage_splits_directions(c);
 }
 
 // The SGS viscosity of one step, on U^n with its ghost layer filled: the
@@ -934,7 +936,7 @@ int step_prelude32(Ctx &c)
     c.step++;
     draw(c);
     launch_ghost(c, c.U);
-    if (!wide_temporal(c)) launch_bface32(c, c.U, c.dist);
+    if (!forms_boundaries(c)) launch_bface32(c, c.U, c.dist);
     return step_sgs(c);
 }
 } // namespace fsl
@@ -1000,8 +1002,16 @@ int fsl_step_phased(fsl_ctx *h, int nsteps)
     return FSL_OK;
 }
 
+// boundary outer states of the fused stage kernels, in the path's precision
+static void launch_faces(Ctx &c, const double *cur)
+{
+    if (c.p.precision == FSL_PREC_FP32) launch_bface32(c, cur, c.dist);
+    else launch_bface(c, cur, c.dist);
+}
+
 // Fused path: per stage a ghost fill, the boundary outer states and one
-// fused stage kernel; stages ping-pong U^n -> Up -> Uq -> U^n.
+// fused stage kernel (kernels that form the boundaries themselves need
+// neither pass between stages); stages ping-pong U^n -> Up -> Uq -> U^n.
 int fsl_step(fsl_ctx *h, int nsteps)
 {
     ApiRange range_("fsl_step");
@@ -1016,57 +1026,37 @@ int fsl_step(fsl_ctx *h, int nsteps)
     if ((rc = slab_check(c, nsteps))) return rc;
     if ((rc = ensure_bf(c))) return rc;
     if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step: the current-stage buffer is not U^n");
-    if (c.p.precision == FSL_PREC_FP32) {
-        if ((rc = ensure_fp32(c))) return rc;
-        const bool wt = wide_temporal(c);
-        // the learned closure's feature velocities: the last stage of a step
-        // writes those of U^{n+1}, so only the first step of a call (whose
-        // U^n the caller may have written) runs the velocity pass
-        float *vel = (wt && c.p.sgs == FSL_SGS_LEARNED && c.cl_alloc) ? c.cl_vel : nullptr;
-        for (int n = 0; n < nsteps; n++) {
-            if (c.co_valid) launch_courant_apply(c);
-            else launch_courant(c);
-            c.step++;
-            draw(c);
-            // U^n's ghost layer: the previous step's last stage wrote it,
-            // unless that step ran before this call
-            if (!wt || n == 0) launch_ghost(c, c.U);
-            if (!wt) launch_bface32(c, c.U, c.dist);
-            c.vel_fresh = vel && n > 0;
-            rc = step_sgs(c);
-            c.vel_fresh = false;
-            if (rc) return rc;
-            if (launch_stage32(c, 1, c.U, c.U, c.Up)) return fail(c, FSL_ERR_CUDA, "FP32 stage kernel");
-            if (!wt) {
-                launch_ghost(c, c.Up);
-                launch_bface32(c, c.Up, c.dist);
-            }
-            launch_stage32(c, 2, c.Up, c.U, c.Uq);
-            if (!wt) {
-                launch_ghost(c, c.Uq);
-                launch_bface32(c, c.Uq, c.dist);
-            }
-            launch_stage32(c, 3, c.Uq, c.U, c.U, true, vel);
-            c.co_valid = true;
-            CKL();
-        }
-        return FSL_OK;
-    }
+    const bool fp32 = c.p.precision == FSL_PREC_FP32;
+    if (fp32 && (rc = ensure_fp32(c))) return rc;
+    const bool fb = forms_boundaries(c);
+    // the learned closure's feature velocities: the last FP32-bulk stage of a
+    // step writes those of U^{n+1}, so only the first step of a call (whose
+    // U^n the caller may have written) runs the velocity pass
+    float *vel = (fp32 && fb && c.p.sgs == FSL_SGS_LEARNED && c.cl_alloc) ? c.cl_vel : nullptr;
     for (int n = 0; n < nsteps; n++) {
         if (c.co_valid) launch_courant_apply(c);
         else launch_courant(c);
         c.step++;
         draw(c);
-        launch_ghost(c, c.U);
-        launch_bface(c, c.U, c.dist);
-        if ((rc = step_sgs(c))) return rc;
-        if (launch_stage(c, 1, c.U, c.U, c.Up)) return fail(c, FSL_ERR_CUDA, "stage kernel attribute");
-        launch_ghost(c, c.Up);
-        launch_bface(c, c.Up, c.dist);
-        launch_stage(c, 2, c.Up, c.U, c.Uq);
-        launch_ghost(c, c.Uq);
-        launch_bface(c, c.Uq, c.dist);
-        launch_stage(c, 3, c.Uq, c.U, c.U, true);
+        // U^n's ghost layer: the previous step's last FP32-bulk stage wrote it,
+        // unless that step ran before this call
+        if (!(fb && fp32) || n == 0) launch_ghost(c, c.U);
+        if (!fb) launch_faces(c, c.U);
+        c.vel_fresh = vel && n > 0;
+        rc = step_sgs(c);
+        c.vel_fresh = false;
+        if (rc) return rc;
+        double *const state[4] = {c.U, c.Up, c.Uq, c.U};
+        for (int s = 1; s <= 3; s++) {
+            double *in = state[s - 1], *out = state[s];
+            if (s > 1 && !fb) {
+                launch_ghost(c, in);
+                launch_faces(c, in);
+            }
+            const int e = fp32 ? launch_stage32(c, s, in, c.U, out, s == 3, s == 3 ? vel : nullptr)
+                               : launch_stage(c, s, in, c.U, out, s == 3);
+            if (e) return fail(c, FSL_ERR_CUDA, "stage kernel");
+        }
         c.co_valid = true;
         CKL();
     }
@@ -1167,6 +1157,7 @@ int fsl_tune(fsl_ctx *h, int key, int value)
     case FSL_TUNE_STAGE_SEG:
         if (value < 1 || value > 1 << 20) return FSL_ERR_ARG;
         c.stage_seg = value;
+        c.seg_set = true;
         return FSL_OK;
     case FSL_TUNE_CLOSURE_POLY:
         if (value < 0 || value > 6 || value == 1) return FSL_ERR_ARG;

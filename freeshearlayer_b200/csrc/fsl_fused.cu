@@ -1,8 +1,9 @@
-// fsl_fused.cu -- FP64 instantiation of the fused stage kernel (the plain
-// method).  Compiled with --fmad=false: every value is formed with the
+// fsl_fused.cu -- FP64 instantiations of the fused stage kernels (the plain
+// method) and the choice between them.  Compiled with --fmad=false: every value is formed with the
 // reference's expressions and rounds exactly like the reference's serial code.
 #define FSL_CHK_UNIT FSL_CHK_FUSED
 #include "fsl_stage.cuh"
+#include "fsl_stage_dir.cuh"
 
 FSL_CHK_EXPORT(fused)
 
@@ -20,6 +21,42 @@ void launch_bface(Ctx &c, const double *cur, const Disturb &d)
     stage::launch_bface_t<double>(c, cur, d, bf64(c));
 }
 
+// How a domain's tiles (tj x tk output cells) are cut along x when one block
+// fits on an SM: the blocks run in waves and a segment of n planes costs n +
+// `start` planes, so take the n whose waves cost least.
+struct Cut {
+    int seg;     // planes per block
+    double cost; // planes one SM marches, starts included
+};
+static Cut cut_tiles(const Grid &g, int sms, int tj, int tk, double start)
+{
+    const long long tiles = (long long)((g.D + tk - 1) / tk) * ((g.H + tj - 1) / tj);
+    Cut best{g.L, -1.};
+    for (int n = 1; n <= g.L; n++) {
+        const long long segs = (g.L + n - 1) / n;
+        const double t = (double)((tiles * segs + sms - 1) / sms) * (n + start);
+        if (best.cost < 0. || t < best.cost) best = {n, t};
+    }
+    return best;
+}
+static Cut ring_cut(const Grid &g, int sms, int tj) { return cut_tiles(g, sms, tj, 30, 1.2); }
+static Cut dir_cut(const Grid &g, int sms) { return cut_tiles(g, sms, dirs::WJ, dirs::WK, 2.0); }
+
+// The ring tile marches a plane of 14 x 30 cells in 11.2 us, the direction-split
+// kernel one of 4 x 32 in 5.1 us and 3 us a launch, whatever the grid (measured
+// from 24x16x16 to 256x128x128): per cell the ring is faster by half, but the
+// smaller tiles leave fewer SMs idle on small grids and no columns empty where
+// DEP is a multiple of 32, and on the temporal setup the direction split needs no
+// boundary passes (18 us a stage).  Per step, ring with its passes against
+// direction split: 64x32x32 197 / 102 us, 512x64x32 1448 / 933, 100x80x35
+// (spatial) 406 / 583, 256x128x128 3431 / 4064.
+bool stage_splits_directions(const Ctx &c)
+{
+    if (c.p.recon != FSL_RECON_CHARMINMOD || c.stage_tje != 0 || c.seg_set) return false;
+    const double passes = c.p.setup == FSL_SETUP_TEMPORAL ? 18. : 0.;
+    return 3. + 5.1 * dir_cut(c.g, c.sms).cost < 11.2 * ring_cut(c.g, c.sms, 14).cost + passes;
+}
+
 template <bool SST>
 static int stage64(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant)
 {
@@ -29,9 +66,15 @@ static int stage64(Ctx &c, int stage, const double *cur, const double *un, doubl
     if (c.p.recon == FSL_RECON_PPM) {
         if (c.stage_tje == 8)
             return stage::launch_stage_t<double, 8, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
-        return stage::launch_stage_t<double, 12, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
+        return stage::launch_stage_t<double, 12, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant,
+                                                               c.stage_tje || c.seg_set ? 0 : ring_cut(c.g, c.sms, 10).seg);
     }
     switch (c.stage_tje) {
+    case 0:
+        if (stage_splits_directions(c))
+            return dirs::launch_stage_dir<SST>(c, stage, cur, un, out, c.mu, bf64(c), courant, dir_cut(c.g, c.sms).seg);
+        return stage::launch_stage_t<double, 16, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant,
+                                                                c.seg_set ? 0 : ring_cut(c.g, c.sms, 14).seg);
     case 8: return stage::launch_stage_t<double, 8, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
     case 12: return stage::launch_stage_t<double, 12, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
     default: return stage::launch_stage_t<double, 16, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);

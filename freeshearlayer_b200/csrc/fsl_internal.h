@@ -92,8 +92,9 @@ struct Ctx {
     BFaces32 bf32{};
     float *mu32 = nullptr;
     bool fp32_alloc = false;
-    int stage_tje = 16; // rows per fused-stage ring tile (incl. the two halo rows); 0: full-lane tile (FP32)
+    int stage_tje = 0; // rows per fused-stage ring tile (incl. the two halo rows); 0: full-lane tile (FP32), by the grid (FP64)
     int stage_seg = 32; // x planes per fused-stage block (fsl_init: 48 for FP32 bulk)
+    bool seg_set = false; // by fsl_tune: FP64 stages with rows 0 then run the 16-row ring tile so cut
     // learned closure
     ClosureScales cls{};
     float *cl_params = nullptr; // FP32 parameter vector (kNParams)
@@ -223,6 +224,8 @@ void launch_plane_sums(Ctx &c, const double *U, int i0, int ni, double *rows);
 void launch_bface(Ctx &c, const double *cur, const Disturb &d);
 // One RK3 stage: cur (ghosts filled) -> out; un = U^n.
 int launch_stage(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant = false);
+// whether launch_stage runs the direction-split kernel (rows 0, small grids)
+bool stage_splits_directions(const Ctx &c);
 // FP32-bulk variants (fsl_fused32.cu): boundary states in bf32, SGS viscosity in mu32.
 void launch_bface32(Ctx &c, const double *cur, const Disturb &d);
 // vel (full-lane tile, temporal setup, stage 3 only): also write the FP32

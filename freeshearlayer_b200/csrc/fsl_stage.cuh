@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
 
 template <typename T, int TJE, int MINB, bool PPM = false, bool SST = false>
 int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, double *out, const T *mu, BF<T> bf,
-                   bool courant)
+                   bool courant, int seg = 0)
 {
     const Grid &g = c.g;
     Args<T> a;
@@ -650,7 +650,7 @@ int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, doubl
     a.co_i0 = c.co_i0;
     a.co_i1 = c.co_i1;
     a.status = &c.ds->status;
-    a.seg = c.stage_seg;
+    a.seg = seg > 0 ? seg : c.stage_seg;
     a.vel = nullptr;
     const size_t smem = sizeof(Smem<T, TJE, PPM>);
     static std::atomic<uint64_t> attr{0};

@@ -307,10 +307,12 @@ int fsl_step_stage(fsl_ctx *ctx);
  * them; FP32-bulk results may differ in the last bits (the compiler may
  * contract a flux into FMAs differently where a block's march starts). */
 #define FSL_TUNE_STAGE_ROWS 1 /* rows per ring stage tile incl. 2 halo rows: 8, 12 or 16; or 0, the
-                                 full-lane persistent 16 x 32 tile (the FP32 bulk's default with the
-                                 reference reconstruction; elsewhere 0 runs 16) */
+                                 default: the full-lane persistent 16 x 32 tile (FP32 bulk with the
+                                 reference reconstruction), 16 (FP32 bulk with PPM), or the kernel and
+                                 the planes per block the grid calls for (FP64) */
 #define FSL_TUNE_STAGE_SEG 2  /* x planes marched per ring-tile stage block (default 48 FP32 bulk, 32 FP64;
-                                 the full-lane tile splits the planes among its blocks itself) */
+                                 with rows 0 the FP32 bulk's full-lane tile splits the planes itself, FP64
+                                 stages run 16 rows once this is set) */
 #define FSL_TUNE_CLOSURE_POLY 3 /* learned-closure inference: of every 8 SiLU value pairs, how many take
                                    the FMA-pipe polynomial tanh instead of the MUFU one: 0 or 2..6
                                    (default 2: 1.94 ms per step at 512x256x256 against 1.97 for 3;
