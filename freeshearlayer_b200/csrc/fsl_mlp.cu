@@ -470,6 +470,8 @@ __global__ void k_harvest(Grid g, ClosureScales sc, const double *__restrict__ U
 // TMEM columns of one training block
 constexpr uint32_t kZ1 = 0, kZ2 = 64, kZ3 = 128, kGW1 = 192, kGW2 = 256, kGW3 = 320, kDG = 384;
 
+constexpr int kTrainThreads = 512; // four per cell of a tile
+
 struct SmemTrain {
     SmemW w;
     alignas(128) __nv_bfloat16 W2T[64 * 64]; // B operand of the data gradient: [in][out]
@@ -484,6 +486,7 @@ struct SmemTrain {
     alignas(128) __nv_bfloat16 DZT[128 * 128]; // dz, [out (64, zero-padded to 128)][cell]
     float gsum[4][4][64];            // per warp: the gradients of b1, b2, b3, w4
     float gone[4][2];                // per warp: the gradient of b4, the loss
+    float ypart[4][128];             // the four threads' parts of a cell's output
     uint64_t mbar;
     uint32_t tholder;
 };
@@ -521,16 +524,17 @@ __device__ __forceinline__ void store_row16(__nv_bfloat16 *A, int t, int c0, con
     }
 }
 
-// This warp's 32 rows of the 128 x 64 tile A (K-major, width 64) into the
-// transposed tile AT (rows = A's columns, width 128): 8 x 8 core matrices
-// through ldmatrix.trans / stmatrix, four at a time.
-__device__ __forceinline__ void transpose_rows(const __nv_bfloat16 *A, __nv_bfloat16 *AT, int wp, int l)
+// This warp's 32 rows x 16 columns (chunk c) of the 128 x 64 tile A (K-major,
+// width 64) into the transposed tile AT (rows = A's columns, width 128): 8 x 8
+// core matrices through ldmatrix.trans / stmatrix, four at a time.
+__device__ __forceinline__ void transpose_chunk(const __nv_bfloat16 *A, __nv_bfloat16 *AT, int wp, int c, int l)
 {
     __syncwarp();
     const uint32_t src = umma::smem_u32(A) + (uint32_t)(wp * 4 + (l >> 3)) * 1024u + (uint32_t)(l & 7) * 16u;
     const uint32_t dst = umma::smem_u32(AT) + (uint32_t)(wp * 4 + (l >> 3)) * 128u + (uint32_t)(l & 7) * 16u;
 #pragma unroll
-    for (uint32_t ob = 0; ob < 8; ob++) {
+    for (uint32_t h = 0; h < 2; h++) {
+        const uint32_t ob = 2u * (uint32_t)c + h;
         uint32_t r0, r1, r2, r3;
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                      : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
@@ -565,12 +569,14 @@ __device__ __forceinline__ float warp_colsum16(const float *in, int l)
 // accumulated per block into Gpart[blockIdx.x][kNParams]; loss_part holds
 // the block's summed squared error.  Each block handles tiles
 // [blockIdx.x * tpb, (blockIdx.x + 1) * tpb).  TMEM (448 of 512 columns) allows
-// one block of four warps per SM, so the chain of seven products and their
-// epilogues bounds it.  The bias, w4 and loss sums are taken over a warp's
-// lanes with shuffles and kept in registers from tile to tile: as atomic adds
-// to one shared word per column they serialised a tile's 128 threads 256
-// times over (a gradient of 2^20 samples: 75 ms then, 0.85 ms now).
-__global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__ X, const float *__restrict__ Yt,
+// one block per SM, so the chain of seven products and their epilogues bounds
+// it; four threads share a cell (a TMEM lane), each with 16 of a layer's 64
+// columns, so that four warps a scheduler hide the epilogues' latency (a
+// gradient of 2^20 samples: 0.85 ms with one thread a cell, 0.51 ms now).  The bias,
+// w4 and loss sums are taken over a warp's lanes with shuffles and kept in
+// registers from tile to tile: as atomic adds to one shared word per column they
+// serialised a tile's cells 256 times over (75 ms).
+__global__ void __launch_bounds__(kTrainThreads, 1) k_train_grad(const float *__restrict__ X, const float *__restrict__ Yt,
                                                        long long n, int tpb, const float *__restrict__ P,
                                                        float *__restrict__ Gpart, float *__restrict__ loss_part,
                                                        int *err, float inv_wmean)
@@ -578,19 +584,20 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
     extern __shared__ __align__(1024) unsigned char smraw[];
     SmemTrain &s = *reinterpret_cast<SmemTrain *>(smraw);
     if (*err) return; // an earlier pass gave up: its caller reports it
-    const int t = threadIdx.x, wp = t >> 5, l = t & 31;
-    stage_weights(s.w, P, t, 128);
-    for (int e = t; e < 64 * 64; e += 128) {
+    // cell (TMEM lane) t of the tile, columns 16 c .. 16 c + 15
+    const int x = threadIdx.x, t = x & 127, c = x >> 7, wp = t >> 5, l = t & 31, c0 = c * 16;
+    stage_weights(s.w, P, x, kTrainThreads);
+    for (int e = x; e < 64 * 64; e += kTrainThreads) {
         const int o = e / 64, i = e % 64; // W[o][i] -> WT[i][o]
         s.W2T[umma::tile_off(i, o, 64) / 2] = __float2bfloat16_rn(P[kOffW2 + e]);
         s.W3T[umma::tile_off(i, o, 64) / 2] = __float2bfloat16_rn(P[kOffW3 + e]);
     }
     // the padding: rows 64..127 of dz^T, inputs 8..15 of the features
-    for (int e = t; e < 128 * 128; e += 128) s.DZT[e] = __float2bfloat16_rn(0.f);
-    for (int e = t; e < 128 * 16; e += 128) s.A0[e] = s.A0T[e] = __float2bfloat16_rn(0.f);
-    if (t == 0) umma::mbar_init(&s.mbar, 1);
-    float gb1[4] = {}, gb2[4] = {}, gb3[4] = {}, gw4[4] = {}, gb4 = 0.f, loss = 0.f;
-    if (wp == 0) umma::tmem_alloc(&s.tholder, 512);
+    for (int e = x; e < 128 * 128; e += kTrainThreads) s.DZT[e] = __float2bfloat16_rn(0.f);
+    for (int e = x; e < 128 * 16; e += kTrainThreads) s.A0[e] = s.A0T[e] = __float2bfloat16_rn(0.f);
+    if (x == 0) umma::mbar_init(&s.mbar, 1);
+    float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, gw4 = 0.f, gb4 = 0.f, loss = 0.f;
+    if (x < 32) umma::tmem_alloc(&s.tholder, 512);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -626,7 +633,7 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         const float f[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
         const float target = yt;
         fetch(tile + 1, tt + 1 < tpb); // the next tile's samples, in flight during this one
-        {
+        if (c == 0) {
             uint32_t p[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -640,52 +647,47 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         }
         // ---- forward: z1, z2, z3 stay in TMEM ----
         sync_for_mma();
-        if (t == 0) { umma::gemm_issue(tmem + kZ1, aA0, aW1, 16, 64, false); umma::commit(&s.mbar); }
+        if (x == 0) { umma::gemm_issue(tmem + kZ1, aA0, aW1, 16, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
         if (!ok) break;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
+        {
             float v[16];
-            umma::tmem_ld16(lane + kZ1 + c * 16, v);
+            umma::tmem_ld16(lane + kZ1 + c0, v);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b1[c * 16 + q]);
-            store_row16(s.A1, t, c * 16, v);
+            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b1[c0 + q]);
+            store_row16(s.A1, t, c0, v);
+            transpose_chunk(s.A1, s.A1T, wp, c, l);
         }
-        transpose_rows(s.A1, s.A1T, wp, l);
         sync_for_mma();
-        if (t == 0) { umma::gemm_issue(tmem + kZ2, aA1, aW2, 64, 64, false); umma::commit(&s.mbar); }
+        if (x == 0) { umma::gemm_issue(tmem + kZ2, aA1, aW2, 64, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
         if (!ok) break;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
+        {
             float v[16];
-            umma::tmem_ld16(lane + kZ2 + c * 16, v);
+            umma::tmem_ld16(lane + kZ2 + c0, v);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b2[c * 16 + q]);
-            store_row16(s.A2, t, c * 16, v);
+            for (int q = 0; q < 16; q++) v[q] = silu(v[q] + s.w.b2[c0 + q]);
+            store_row16(s.A2, t, c0, v);
+            transpose_chunk(s.A2, s.A2T, wp, c, l);
         }
-        transpose_rows(s.A2, s.A2T, wp, l);
         sync_for_mma();
-        if (t == 0) { umma::gemm_issue(tmem + kZ3, aA2, aW3, 64, 64, false); umma::commit(&s.mbar); }
+        if (x == 0) { umma::gemm_issue(tmem + kZ3, aA2, aW3, 64, 64, false); umma::commit(&s.mbar); }
         mma_wait(s, phase, ok);
         if (!ok) break;
         // ---- output, loss gradient, layer 3 backward ----
-        float z3[64];
-        float y = s.w.b4;
+        float z3[16], y = 0.f;
+        umma::tmem_ld16(lane + kZ3 + c0, z3);
+        umma::tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            float v[16];
-            umma::tmem_ld16(lane + kZ3 + c * 16, v);
-            umma::tmem_wait_ld();
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int o = c * 16 + q;
-                z3[o] = v[q] + s.w.b3[o];
-                y += s.w.w4[o] * silu(z3[o]);
-            }
+        for (int q = 0; q < 16; q++) {
+            z3[q] += s.w.b3[c0 + q];
+            y += s.w.w4[c0 + q] * silu(z3[q]);
         }
+        s.ypart[c][t] = y;
+        __syncthreads();
+        y = s.w.b4 + s.ypart[0][t] + s.ypart[1][t] + s.ypart[2][t] + s.ypart[3][t];
         // sample weight: 1, or (rho |S| t_ref)^2 over its dataset mean, which
         // makes the loss the squared error of mu_SGS = rho Cs^2 DD |S|
         float wgt = 1.f;
@@ -695,125 +697,124 @@ __global__ void __launch_bounds__(128, 1) k_train_grad(const float *__restrict__
         }
         const float e = valid ? (y - target) : 0.f;
         const float dy = scale * wgt * e;
-        loss += wgt * e * e;
-        gb4 += dy;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
+        if (c == 0) {
+            loss += wgt * e * e;
+            gb4 += dy;
+        }
+        {
             float v[16], g4[16];
 #pragma unroll
             for (int q = 0; q < 16; q++) {
-                const float z = z3[c * 16 + q];
-                g4[q] = dy * silu(z);
-                v[q] = dy * s.w.w4[c * 16 + q] * dsilu(z);
+                g4[q] = dy * silu(z3[q]);
+                v[q] = dy * s.w.w4[c0 + q] * dsilu(z3[q]);
             }
-            gw4[c] += warp_colsum16(g4, l);
-            gb3[c] += warp_colsum16(v, l);
-            store_row16(s.DZ, t, c * 16, v);
+            gw4 += warp_colsum16(g4, l);
+            gb3 += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c0, v);
+            transpose_chunk(s.DZ, s.DZT, wp, c, l);
         }
-        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW3 += dz3^T a2 ; da2 = dz3 W3
         sync_for_mma();
-        if (t == 0) {
+        if (x == 0) {
             umma::gemm_issue(tmem + kGW3, aDZT, aA2T, 128, 64, acc);
             umma::gemm_issue(tmem + kDG, aDZ, aW3T, 64, 64, false);
             umma::commit(&s.mbar);
         }
         mma_wait(s, phase, ok);
         if (!ok) break;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
+        {
             float v[16], zz[16];
-            umma::tmem_ld16(lane + kDG + c * 16, v);
-            umma::tmem_ld16(lane + kZ2 + c * 16, zz);
+            umma::tmem_ld16(lane + kDG + c0, v);
+            umma::tmem_ld16(lane + kZ2 + c0, zz);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b2[c * 16 + q]) : 0.f;
-            gb2[c] += warp_colsum16(v, l);
-            store_row16(s.DZ, t, c * 16, v);
+            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b2[c0 + q]) : 0.f;
+            gb2 += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c0, v);
+            transpose_chunk(s.DZ, s.DZT, wp, c, l);
         }
-        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW2 += dz2^T a1 ; da1 = dz2 W2
         sync_for_mma();
-        if (t == 0) {
+        if (x == 0) {
             umma::gemm_issue(tmem + kGW2, aDZT, aA1T, 128, 64, acc);
             umma::gemm_issue(tmem + kDG, aDZ, aW2T, 64, 64, false);
             umma::commit(&s.mbar);
         }
         mma_wait(s, phase, ok);
         if (!ok) break;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
+        {
             float v[16], zz[16];
-            umma::tmem_ld16(lane + kDG + c * 16, v);
-            umma::tmem_ld16(lane + kZ1 + c * 16, zz);
+            umma::tmem_ld16(lane + kDG + c0, v);
+            umma::tmem_ld16(lane + kZ1 + c0, zz);
             umma::tmem_wait_ld();
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b1[c * 16 + q]) : 0.f;
-            gb1[c] += warp_colsum16(v, l);
-            store_row16(s.DZ, t, c * 16, v);
+            for (int q = 0; q < 16; q++) v[q] = valid ? v[q] * dsilu(zz[q] + s.w.b1[c0 + q]) : 0.f;
+            gb1 += warp_colsum16(v, l);
+            store_row16(s.DZ, t, c0, v);
+            transpose_chunk(s.DZ, s.DZT, wp, c, l);
         }
-        transpose_rows(s.DZ, s.DZT, wp, l);
         // dW1 += dz1^T a0
         sync_for_mma();
-        if (t == 0) {
+        if (x == 0) {
             umma::gemm_issue(tmem + kGW1, aDZT, aA0T, 128, 16, acc);
             umma::commit(&s.mbar);
         }
         mma_wait(s, phase, ok);
         if (!ok) break;
     }
-    // the warps' sums to shared memory (lanes 0..15 hold a chunk's 16 columns)
+    // the warps' sums to shared memory (lanes 0..15 hold the chunk's 16 columns)
     if (l < 16) {
+        s.gsum[wp][0][c0 + l] = gb1;
+        s.gsum[wp][1][c0 + l] = gb2;
+        s.gsum[wp][2][c0 + l] = gb3;
+        s.gsum[wp][3][c0 + l] = gw4;
+    }
+    if (c == 0) {
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            s.gsum[wp][0][c * 16 + l] = gb1[c];
-            s.gsum[wp][1][c * 16 + l] = gb2[c];
-            s.gsum[wp][2][c * 16 + l] = gb3[c];
-            s.gsum[wp][3][c * 16 + l] = gw4[c];
+        for (int o = 16; o > 0; o >>= 1) {
+            loss += __shfl_xor_sync(0xffffffffu, loss, o);
+            gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
         }
+        if (l == 0) { s.gone[wp][0] = gb4; s.gone[wp][1] = loss; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        loss += __shfl_xor_sync(0xffffffffu, loss, o);
-        gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
-    }
-    if (l == 0) { s.gone[wp][0] = gb4; s.gone[wp][1] = loss; }
     // ---- block partial gradients ----
     float *G = Gpart + (long long)blockIdx.x * kNParams;
     if (ok) {
         if (wp < 2) { // TMEM lanes 0..63 hold the weight-gradient rows (output features)
             const int o = t;
-            for (int c = 0; c < 4; c++) {
-                float v[16];
-                umma::tmem_ld16(lane + kGW2 + c * 16, v);
-                umma::tmem_wait_ld();
-                for (int q = 0; q < 16; q++) G[kOffW2 + o * 64 + c * 16 + q] = v[q];
-                umma::tmem_ld16(lane + kGW3 + c * 16, v);
-                umma::tmem_wait_ld();
-                for (int q = 0; q < 16; q++) G[kOffW3 + o * 64 + c * 16 + q] = v[q];
-            }
             float v[16];
-            umma::tmem_ld16(lane + kGW1, v);
+            umma::tmem_ld16(lane + kGW2 + c0, v);
             umma::tmem_wait_ld();
-            for (int q = 0; q < 16; q++) G[kOffW1 + o * 16 + q] = (q < 8) ? v[q] : 0.f;
+#pragma unroll
+            for (int q = 0; q < 16; q++) G[kOffW2 + o * 64 + c0 + q] = v[q];
+            umma::tmem_ld16(lane + kGW3 + c0, v);
+            umma::tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 16; q++) G[kOffW3 + o * 64 + c0 + q] = v[q];
+            if (c == 0) {
+                umma::tmem_ld16(lane + kGW1, v);
+                umma::tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < 16; q++) G[kOffW1 + o * 16 + q] = (q < 8) ? v[q] : 0.f;
+            }
         }
         __syncthreads();
-        for (int e = t; e < 4 * 64; e += 128) {
+        for (int e = x; e < 4 * 64; e += kTrainThreads) {
             const int which = e >> 6, o = e & 63;
             const int at = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
             G[at + o] = s.gsum[0][which][o] + s.gsum[1][which][o] + s.gsum[2][which][o] + s.gsum[3][which][o];
         }
-        if (t == 0) {
+        if (x == 0) {
             G[kOffB4] = s.gone[0][0] + s.gone[1][0] + s.gone[2][0] + s.gone[3][0];
             loss_part[blockIdx.x] = s.gone[0][1] + s.gone[1][1] + s.gone[2][1] + s.gone[3][1];
         }
     } else {
-        if (t == 0) atomicExch(err, 1);
+        if (x == 0) atomicExch(err, 1);
         umma::mbar_wait(&s.mbar, phase ^ 1u, kWaitLimit);
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (wp == 0) umma::tmem_free(tmem, 512);
+    if (x < 32) umma::tmem_free(tmem, 512);
 }
 
 // Deterministic sum of the block partials and an Adam step (FP32 master
@@ -920,7 +921,7 @@ int launch_train_grad(cudaStream_t st, const float *X, const float *Y, long long
     if (!smem_limit_once((const void *)mlp::k_train_grad, smem, attr)) return -1;
     const long long ntile = (n + 127) / 128;
     const int nblk = (int)((ntile + tpb - 1) / tpb);
-    mlp::k_train_grad<<<nblk, 128, smem, st>>>(X, Y, n, tpb, P, Gpart, loss_part, err, inv_wmean);
+    mlp::k_train_grad<<<nblk, mlp::kTrainThreads, smem, st>>>(X, Y, n, tpb, P, Gpart, loss_part, err, inv_wmean);
     *nblk_out = nblk;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
