@@ -83,6 +83,61 @@ template <typename T> FSL_HD void minmod_pair(T a, T b, T &ab, T &ba)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Correctly rounded FP64 reciprocals and quotients without branches (device).
+// The FP64 stage's time goes with its IEEE divisions (53 a cell): each expands
+// into a guarded sequence whose branch cuts the compiler's schedule, so that the
+// chains of a face's divisions do not overlap.  Here the range is checked once for
+// a whole group (a face's Riemann solve, a cell's primitives) and quotients by one
+// denominator share its reciprocal.
+//
+// rcp_rn: Newton's iteration from the gross reciprocal (20 bits); the last step,
+// from within an ulp, gives the rounded reciprocal unless b's significand is all
+// ones (Markstein, IBM J. Res. Dev. 34 (1990) 111).  (Two steps would do for a
+// quotient unless b lies just below a power of two -- as densities near 1 do.)
+//
+// quot_rn: a y corrected twice by its exact remainder a - b q.  After the first
+// correction q is within 1/2 + 2^-52 ulp of a/b, so before its rounding the second
+// is off by at most (1/2 + 2^-52) |b y - 1| ulp, |b y - 1| <= 2^-54 m with m the
+// significand of b in [1, 2); a/b lies at least 2^-53 / m ulp from a midpoint of two
+// doubles (its numerator there is a nonzero integer over 2 b), so the rounding is
+// right for every significand but all ones.  No step may leave the normal range.
+// The callers check both (range_ok, zero_or_range_ok, ones) and divide otherwise;
+// quot_signed also keeps the sign of a zero numerator.
+// ---------------------------------------------------------------------------
+#ifdef __CUDACC__
+__device__ __forceinline__ double rcp_rn(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+}
+__device__ __forceinline__ double quot_rn(double a, double b, double y)
+{
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ double quot_signed(double a, double b, double y)
+{
+    const double q = quot_rn(a, b, y);
+    const int sign = (__double2hiint(a) ^ __double2hiint(b)) & 0x80000000;
+    return __hiloint2double(__double2hiint(q) | sign, __double2loint(q));
+}
+// positive and in [2^-60, 2^60)
+__device__ __forceinline__ bool range_ok(double x) { return (unsigned)(__double2hiint(x) - 0x3c300000) < 0x07800000u; }
+// zero, or of magnitude in [2^-512, 2^120)
+__device__ __forceinline__ bool zero_or_range_ok(double x)
+{
+    const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return u < 0x47700000u && u - 1u >= 0x1fefffffu;
+}
+// a significand whose low word is all ones
+__device__ __forceinline__ bool ones(double x) { return __double2loint(x) == -1; }
+#endif
+
 // Per-cell quantities shared by the three sweeps (src/reconstruction.c:63-88,
 // :104, :142-145).
 template <typename T> struct CellC {
@@ -95,7 +150,7 @@ template <typename T> struct CellC {
 
 // What costs divisions and the square root: velocities, sound speed, 1/(2C)
 // and 1/(2C)/C, from the conserved state c.u.
-template <typename T> FSL_HD void cell_roots(CellC<T> &c)
+template <typename T> FSL_HD void cell_roots_div(CellC<T> &c)
 {
     typedef Kc<T> k;
     T R = T(1.) / c.u[0];
@@ -106,6 +161,47 @@ template <typename T> FSL_HD void cell_roots(CellC<T> &c)
     c.C = sqrt(k::K * P * R);
     c.ll = T(1.) / (c.C + c.C);
     c.ee = c.ll / c.C;
+}
+
+#ifdef __CUDACC__
+struct Roots64 {
+    double U, V, W, C, ll, ee;
+};
+__device__ __noinline__ inline Roots64 cell_roots_by_division(double u0, double u1, double u2, double u3, double u4)
+{
+    CellC<double> c;
+    c.u[0] = u0; c.u[1] = u1; c.u[2] = u2; c.u[3] = u3; c.u[4] = u4;
+    cell_roots_div(c);
+    return Roots64{c.U, c.V, c.W, c.C, c.ll, c.ee};
+}
+// the same values from R = rcp_rn(c.u[0]); 1/(C+C) is half of the rounded 1/C
+__device__ __forceinline__ void cell_roots64(CellC<double> &c, double R)
+{
+    typedef Kc<double> k;
+    c.U = c.u[1] * R;
+    c.V = c.u[2] * R;
+    c.W = c.u[3] * R;
+    const double P = (c.u[4] - 0.5 * (c.u[1] * c.u[1] + c.u[2] * c.u[2] + c.u[3] * c.u[3]) * R) * k::K_1;
+    c.C = sqrt(k::K * P * R);
+    const double y = rcp_rn(c.C);
+    c.ll = 0.5 * y;
+    c.ee = quot_rn(c.ll, c.C, y);
+    if (!range_ok(c.u[0]) || !range_ok(P) || ones(c.u[0]) || ones(c.C)) {
+        const Roots64 o = cell_roots_by_division(c.u[0], c.u[1], c.u[2], c.u[3], c.u[4]);
+        c.U = o.U; c.V = o.V; c.W = o.W; c.C = o.C; c.ll = o.ll; c.ee = o.ee;
+    }
+}
+#endif
+
+template <typename T> FSL_HD void cell_roots(CellC<T> &c)
+{
+#ifdef __CUDA_ARCH__
+    if constexpr (std::is_same<T, double>::value) {
+        cell_roots64(c, rcp_rn(c.u[0]));
+        return;
+    }
+#endif
+    cell_roots_div(c);
 }
 
 // The products of those.
@@ -455,7 +551,7 @@ FSL_HD void ppm_z(const CellC<T> &c, const T *m2, const T *m1, const T *p1, cons
 // conserved states.  Returns interface density, pressure and velocity (the
 // normal component from the solve, the tangential ones upwinded by its sign).
 template <typename T, int N>
-FSL_HD void riemann(const T *Lm, const T *Rp, T &Rho, T &Pr, T *vel)
+FSL_HD void riemann_div(const T *Lm, const T *Rp, T &Rho, T &Pr, T *vel)
 {
     typedef Kc<T> k;
     T _R, _P, _C, _jo, _jp, _jm, RU, R_, P_, C_, jo_, jp_, jm_;
@@ -499,6 +595,94 @@ FSL_HD void riemann(const T *Lm, const T *Rp, T &Rho, T &Pr, T *vel)
     vel[N - 1] = Un;
 }
 
+#ifdef __CUDACC__
+struct Riemann64 {
+    double Rho, P, v0, v1, v2;
+};
+template <int N>
+__device__ __noinline__ Riemann64 riemann_by_division(double l0, double l1, double l2, double l3, double l4, double r0,
+                                                      double r1, double r2, double r3, double r4)
+{
+    const double Lm[5] = {l0, l1, l2, l3, l4}, Rp[5] = {r0, r1, r2, r3, r4};
+    double Rho, P, v[3];
+    riemann_div<double, N>(Lm, Rp, Rho, P, v);
+    return Riemann64{Rho, P, v[0], v[1], v[2]};
+}
+// One side of the solve with shared reciprocals; p, q, r: the squares of the
+// velocities in the order their sum takes.  false: divide instead.
+__device__ __forceinline__ bool riemann_side64(double R, double m0, double m1, double m2, double &v0, double &v1,
+                                               double &v2, double &y)
+{
+    y = rcp_rn(R);
+    v0 = quot_signed(m0, R, y);
+    v1 = quot_signed(m1, R, y);
+    v2 = quot_signed(m2, R, y);
+    return range_ok(R) && !ones(R) && zero_or_range_ok(m0) && zero_or_range_ok(m1) && zero_or_range_ok(m2);
+}
+__device__ __forceinline__ bool riemann_side64(double R, double P, double y, double &C, double &RU)
+{
+    C = sqrt(quot_rn(Kc<double>::K * P, R, y));
+    const double RC = R * C;
+    RU = quot_rn(P, RC, rcp_rn(RC));
+    return range_ok(P) && !ones(RC);
+}
+// The upwinded middle of the solve (src/fluxes.c:85-113) from both sides' n
+// velocity, P, C and RU.  With the sides' ranges checked every quotient here is
+// normal or of a zero numerator; false: divide instead.
+__device__ __forceinline__ bool riemann_mid64(double ln, double lP, double lC, double lRU, double rn, double rP,
+                                              double rC, double rRU, double &Rho, double &P, double &vn)
+{
+    typedef Kc<double> k;
+    const double ljo = k::NK_1 * lP, ljp = ln + lRU, ljm = ln - lRU;
+    const double rjo = k::NK_1 * rP, rjp = rn + rRU, rjm = rn - rRU;
+    const double Un = 0.5 * (ln + rn), C = 0.5 * (lC + rC);
+    const bool pp = Un + C > 0., pm = Un - C > 0., po = Un > 0.;
+    const double bp = pp ? ljo : rjo, bm = pm ? ljo : rjo;
+    const double al_p = quot_rn(k::K_1_2 * (pp ? (ljm - ljp) : (rjm - rjp)), bp, rcp_rn(bp));
+    const double al_m = quot_rn(k::K_1_2 * (pm ? (ljp - ljm) : (rjp - rjm)), bm, rcp_rn(bm));
+    const double Jp = pp ? ljp : rjp, Jm = pm ? ljm : rjm, Jo = po ? ljo : rjo;
+    double al_o = k::K05 * (po ? (ljp - ljm) : (rjp - rjm));
+    al_o = -al_o * al_o;
+    const double da = al_p - al_m;
+    P = quot_rn(Jp - Jm, da, rcp_rn(da));
+    vn = Jp - al_p * P;
+    Rho = quot_rn(Jo - P, al_o, rcp_rn(al_o));
+    return !(ones(bp) || ones(bm) || ones(da) || ones(al_o));
+}
+#endif
+
+template <typename T, int N>
+FSL_HD void riemann(const T *Lm, const T *Rp, T &Rho, T &Pr, T *vel)
+{
+#ifdef __CUDA_ARCH__
+    if constexpr (std::is_same<T, double>::value) {
+        typedef Kc<double> k;
+        double l[3], r[3], ly, ry, lC, lRU, rC, rRU;
+        bool ok = riemann_side64(Lm[0], Lm[1], Lm[2], Lm[3], l[0], l[1], l[2], ly);
+        ok = riemann_side64(Rp[0], Rp[1], Rp[2], Rp[3], r[0], r[1], r[2], ry) && ok;
+        const double lP = (Lm[4] - 0.5 * Lm[0] * (l[0] * l[0] + l[1] * l[1] + l[2] * l[2])) * k::K_1;
+        const double rP = (Rp[4] - 0.5 * Rp[0] * (r[0] * r[0] + r[1] * r[1] + r[2] * r[2])) * k::K_1;
+        ok = riemann_side64(Lm[0], lP, ly, lC, lRU) && ok;
+        ok = riemann_side64(Rp[0], rP, ry, rC, rRU) && ok;
+        double vn;
+        ok = riemann_mid64(l[N - 1], lP, lC, lRU, r[N - 1], rP, rC, rRU, Rho, Pr, vn) && ok;
+        const bool up = vn > 0.;
+        vel[0] = up ? l[0] : r[0];
+        vel[1] = up ? l[1] : r[1];
+        vel[2] = up ? l[2] : r[2];
+        vel[N - 1] = vn;
+        if (!ok) {
+            const Riemann64 o = riemann_by_division<N>(Lm[0], Lm[1], Lm[2], Lm[3], Lm[4], Rp[0], Rp[1], Rp[2], Rp[3],
+                                                       Rp[4]);
+            Rho = o.Rho; Pr = o.P;
+            vel[0] = o.v0; vel[1] = o.v1; vel[2] = o.v2;
+        }
+        return;
+    }
+#endif
+    riemann_div<T, N>(Lm, Rp, Rho, Pr, vel);
+}
+
 // Velocities by reciprocal, RU = 1./rho (src/fluxes.c:124-142).
 template <typename T> FSL_HD void vel_rcp(T r, T mu_, T mv, T mw, T *o)
 {
@@ -507,13 +691,56 @@ template <typename T> FSL_HD void vel_rcp(T r, T mu_, T mv, T mw, T *o)
 }
 
 // Velocities and temperature by division (src/fluxes.c:117-122).
-template <typename T> FSL_HD void vel_div(T R_, T mu_, T mv, T mw, T E, T *o, T &Tt)
+template <typename T> FSL_HD void vel_div_div(T R_, T mu_, T mv, T mw, T E, T *o, T &Tt)
 {
     typedef Kc<T> k;
     T U_ = mu_ / R_, V_ = mv / R_, W_ = mw / R_;
     T P_ = (E - T(0.5) * R_ * (U_ * U_ + V_ * V_ + W_ * W_)) * k::K_1;
     Tt = P_ / (k::R_VOZD * R_);
     o[0] = U_; o[1] = V_; o[2] = W_;
+}
+
+#ifdef __CUDACC__
+struct VelT64 {
+    double u, v, w, T;
+};
+__device__ __noinline__ inline VelT64 vel_by_division(double R, double m0, double m1, double m2, double E)
+{
+    VelT64 o;
+    double v[3];
+    vel_div_div(R, m0, m1, m2, E, v, o.T);
+    o.u = v[0]; o.v = v[1]; o.w = v[2];
+    return o;
+}
+// the same values; y = rcp_rn(R)
+__device__ __forceinline__ void vel_div64(double R, double m0, double m1, double m2, double E, double y, double *o,
+                                          double &Tt)
+{
+    typedef Kc<double> k;
+    o[0] = quot_signed(m0, R, y);
+    o[1] = quot_signed(m1, R, y);
+    o[2] = quot_signed(m2, R, y);
+    const double P = (E - 0.5 * R * (o[0] * o[0] + o[1] * o[1] + o[2] * o[2])) * k::K_1;
+    const double den = k::R_VOZD * R;
+    Tt = quot_rn(P, den, rcp_rn(den));
+    if (!(range_ok(R) && range_ok(P) && zero_or_range_ok(m0) && zero_or_range_ok(m1) && zero_or_range_ok(m2)) ||
+        ones(R) || ones(den)) {
+        const VelT64 q = vel_by_division(R, m0, m1, m2, E);
+        o[0] = q.u; o[1] = q.v; o[2] = q.w;
+        Tt = q.T;
+    }
+}
+#endif
+
+template <typename T> FSL_HD void vel_div(T R_, T mu_, T mv, T mw, T E, T *o, T &Tt)
+{
+#ifdef __CUDA_ARCH__
+    if constexpr (std::is_same<T, double>::value) {
+        vel_div64(R_, mu_, mv, mw, E, rcp_rn(R_), o, Tt);
+        return;
+    }
+#endif
+    vel_div_div(R_, mu_, mv, mw, E, o, Tt);
 }
 
 // Flux assembly of one face from the Riemann state, the face velocity
@@ -608,6 +835,17 @@ template <typename T> FSL_HD void vdiv(const T *U, T *o)
     vel_div(U[0], U[1], U[2], U[3], U[4], o, Tt);
     o[3] = Tt;
 }
+
+#ifdef __CUDACC__
+// A cell's characteristic roots and its velocities and temperature by division
+// (dv), sharing 1/rho.
+__device__ __forceinline__ void cell_prims64(CellC<double> &c, double *dv)
+{
+    const double y = rcp_rn(c.u[0]);
+    cell_roots64(c, y);
+    vel_div64(c.u[0], c.u[1], c.u[2], c.u[3], c.u[4], y, dv, dv[3]);
+}
+#endif
 
 // Courant number of one cell from its conserved variables: the reference's
 // streamwise u dt/dx (src/helpers.c:31-43) or the acoustic sum

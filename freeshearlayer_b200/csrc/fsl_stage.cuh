@@ -160,9 +160,15 @@ __global__ void k_bface(Grid g, int setup, int BL_HIG, Disturb d, const double *
 
 template <typename T, int TJE, bool PPM = false> struct Smem {
     static constexpr int HW = PPM ? 2 : 1; // y/z halo width of the state planes
-    static constexpr int NS = PPM ? 4 : 2; // x-planes in the state ring
-    // current-stage state: planes i, i+1 (PPM: i-1 .. i+2) as a ring, with
-    // HW halo rows and lanes
+    // FP64 planes arrive in shared memory by asynchronous copies, into a slot of
+    // their own (in registers, as the FP32 bulk's conversion needs them, a plane in
+    // flight costs 20 of the 128 a thread has); FP32 planes replace a slot whose
+    // readers are done
+    static constexpr bool ASYNC = sizeof(T) == 8;
+    static constexpr int NS = (PPM ? 4 : 2) + (ASYNC ? 1 : 0); // x-planes in the state ring
+    __device__ static __forceinline__ int slot(int p) { return ASYNC ? (p + NS) % NS : p & (NS - 1); }
+    // current-stage state: planes i, i+1 (PPM: i-1 .. i+2; FP64: and the next) as
+    // a ring, with HW halo rows and lanes
     T U[NS][TJE + 2 * HW][32 + 2 * HW][5];
     T R[3][TJE][32][3];     // velocities by reciprocal, planes i-1, i, i+1 (ring)
     T Dv[2][TJE][32][5];    // velocities by division, temperature, mu face average, planes i, i+1
@@ -200,26 +206,46 @@ struct PlaneLoad {
     double own[5], halo[5], halo2[5]; // halo2: the second halo cell (PPM)
 };
 
-template <typename T, int TJE, bool PPM>
-__device__ __forceinline__ void plane_issue(const Grid &g, const double *__restrict__ cu, int pl, int r, int l, int j,
-                                            int k, bool live, PlaneLoad &p)
+// FP64: straight into the plane's ring slot; else into registers.
+__device__ __forceinline__ void copy5_async(double *dst, const double *__restrict__ u, long long fs, long long c)
 {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const double *src = u + FSL_CELL(c, fs);
+#pragma unroll
+    for (int q = 0; q < 5; q++)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + q * 8u), "l"(src + q * fs) : "memory");
+}
+__device__ __forceinline__ void copies_done()
+{
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+template <typename T, int TJE, bool PPM>
+__device__ __forceinline__ void plane_issue(Smem<T, TJE, PPM> &s, const Grid &g, const double *__restrict__ cu, int pl,
+                                            int r, int l, int j, int k, bool live, PlaneLoad &p)
+{
+    constexpr int HW = Smem<T, TJE, PPM>::HW;
     const long long fs = g.fstride;
     if (!live || pl > g.L + 1) return;
     const long long c = g.idx(pl, j, k);
-    load5(cu, fs, c, p.own);
+    auto get = [&](double *reg, int rr, int ll, long long cell) {
+        if constexpr (Smem<T, TJE, PPM>::ASYNC)
+            copy5_async(s.U[Smem<T, TJE, PPM>::slot(pl)][rr][ll], cu, fs, cell);
+        else load5(cu, fs, cell, reg);
+    };
+    get(p.own, r + HW, l + HW, c);
     if (r == 0 && j >= 1) {
-        load5(cu, fs, c - g.pk, p.halo);
-        if (PPM && j >= 2) load5(cu, fs, c - 2 * g.pk, p.halo2);
+        get(p.halo, HW - 1, l + HW, c - g.pk);
+        if (PPM && j >= 2) get(p.halo2, 0, l + HW, c - 2 * g.pk);
     } else if (r == TJE - 1 && j <= g.H) {
-        load5(cu, fs, c + g.pk, p.halo);
-        if (PPM && j <= g.H - 1) load5(cu, fs, c + 2 * g.pk, p.halo2);
+        get(p.halo, TJE + HW, l + HW, c + g.pk);
+        if (PPM && j <= g.H - 1) get(p.halo2, TJE + HW + 1, l + HW, c + 2 * g.pk);
     } else if (l == 0 && k >= 1) {
-        load5(cu, fs, c - 1, p.halo);
-        if (PPM && k >= 2) load5(cu, fs, c - 2, p.halo2);
+        get(p.halo, r + HW, HW - 1, c - 1);
+        if (PPM && k >= 2) get(p.halo2, r + HW, 0, c - 2);
     } else if (l == 31 && k <= g.D) {
-        load5(cu, fs, c + 1, p.halo);
-        if (PPM && k <= g.D - 1) load5(cu, fs, c + 2, p.halo2);
+        get(p.halo, r + HW, 32 + HW, c + 1);
+        if (PPM && k <= g.D - 1) get(p.halo2, r + HW, 33 + HW, c + 2);
     }
 }
 
@@ -228,6 +254,7 @@ __device__ __forceinline__ void plane_store(Smem<T, TJE, PPM> &s, int slot, int 
                                             bool live, const PlaneLoad &p)
 {
     constexpr int HW = Smem<T, TJE, PPM>::HW;
+    if constexpr (Smem<T, TJE, PPM>::ASYNC) return; // already there
     if (!live) return;
 #pragma unroll
     for (int q = 0; q < 5; q++) s.U[slot][r + HW][l + HW][q] = T(p.own[q]);
@@ -260,21 +287,21 @@ __device__ __forceinline__ void plane_store(Smem<T, TJE, PPM> &s, int slot, int 
 template <typename T, int TJE, bool PPM, bool SST>
 __device__ __forceinline__ void plane_prims(Smem<T, TJE, PPM> &s, int pl, int r, int l, T mu_pl, T mu_prev)
 {
-    constexpr int HW = Smem<T, TJE, PPM>::HW, NS = Smem<T, TJE, PPM>::NS;
-    const T *u = s.U[pl & (NS - 1)][r + HW][l + HW];
+    constexpr int HW = Smem<T, TJE, PPM>::HW;
+    const T *u = s.U[Smem<T, TJE, PPM>::slot(pl)][r + HW][l + HW];
+    T dv[4];
     if constexpr (Smem<T, TJE, PPM>::ROOTS) {
         CellC<T> c;
 #pragma unroll
         for (int q = 0; q < 5; q++) c.u[q] = u[q];
-        cell_roots(c); // U, V, W are the reciprocal velocities of vel_rcp
+        cell_prims64(c, dv); // U, V, W are the reciprocal velocities of vel_rcp
         T *v = s.R[pl % 3][r][l], *k = s.C[pl & 1][r][l];
         v[0] = c.U; v[1] = c.V; v[2] = c.W;
         k[0] = c.C; k[1] = c.ll; k[2] = c.ee;
     } else {
         vel_rcp(u[0], u[1], u[2], u[3], s.R[pl % 3][r][l]);
+        vdiv(u, dv);
     }
-    T dv[4];
-    vdiv(u, dv);
     T *o = s.Dv[pl & 1][r][l];
     o[0] = dv[0]; o[1] = dv[1]; o[2] = dv[2]; o[3] = dv[3];
     if constexpr (!SST) o[4] = T(0.5) * (mu_pl + mu_prev);
@@ -305,7 +332,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     extern __shared__ __align__(16) unsigned char smraw[];
     typedef Smem<T, TJE, PPM> SM;
     SM &s = *reinterpret_cast<SM *>(smraw);
-    constexpr int HW = SM::HW, NS = SM::NS;
+    constexpr int HW = SM::HW;
     const int L = g.L, H = g.H, D = g.D;
     constexpr int TJ = TJE - 2;
     const int r = threadIdx.y, l = threadIdx.x;
@@ -337,20 +364,21 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     // ---- prologue: planes i0-1 .. i0+1 (PPM: .. i0+2), flux of face i0 - 1/2 ----
     {
         T Um[5] = {0, 0, 0, 0, 0}, mum = 0;
-        plane_issue<T, TJE, PPM>(g, cu, i0, r, l, j, k, live, pl);
-        plane_store<T, TJE, PPM>(s, i0 & (NS - 1), r, l, j, k, H, D, live, pl);
-        plane_issue<T, TJE, PPM>(g, cu, i0 + 1, r, l, j, k, live, pl);
-        plane_store<T, TJE, PPM>(s, (i0 + 1) & (NS - 1), r, l, j, k, H, D, live, pl);
+        plane_issue<T, TJE, PPM>(s, g, cu, i0, r, l, j, k, live, pl);
+        plane_store<T, TJE, PPM>(s, SM::slot(i0), r, l, j, k, H, D, live, pl);
+        plane_issue<T, TJE, PPM>(s, g, cu, i0 + 1, r, l, j, k, live, pl);
+        plane_store<T, TJE, PPM>(s, SM::slot(i0 + 1), r, l, j, k, H, D, live, pl);
         if constexpr (PPM) {
-            plane_issue<T, TJE, PPM>(g, cu, i0 + 2, r, l, j, k, live, pl);
-            plane_store<T, TJE, PPM>(s, (i0 + 2) & (NS - 1), r, l, j, k, H, D, live && i0 + 2 <= L + 1, pl);
+            plane_issue<T, TJE, PPM>(s, g, cu, i0 + 2, r, l, j, k, live, pl);
+            plane_store<T, TJE, PPM>(s, SM::slot(i0 + 2), r, l, j, k, H, D, live && i0 + 2 <= L + 1, pl);
         }
+        if constexpr (SM::ASYNC) copies_done(); // the own cell's copies; the barrier below shows the others'
         if (live) {
             load5(cu, fs, cj + (long long)(i0 - 1) * g.pi, Um);
             if constexpr (PPM) {
                 // plane i0-1 (own column): the x sweep of cell i0+1 reads it
 #pragma unroll
-                for (int q = 0; q < 5; q++) s.U[(i0 - 1) & (NS - 1)][r + HW][l + HW][q] = Um[q];
+                for (int q = 0; q < 5; q++) s.U[SM::slot(i0 - 1)][r + HW][l + HW][q] = Um[q];
             }
             vel_rcp(Um[0], Um[1], Um[2], Um[3], s.R[(i0 - 1) % 3][r][l]);
             if constexpr (!SST) {
@@ -364,7 +392,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
         __syncthreads();
         if (inter) {
             T hm[5], lo[5], hin[5], dm[4], tmp[5];
-            const T *Uc = s.U[i0 & (NS - 1)][r + HW][l + HW], *Un = s.U[(i0 + 1) & (NS - 1)][r + HW][l + HW];
+            const T *Uc = s.U[SM::slot(i0)][r + HW][l + HW], *Un = s.U[SM::slot(i0 + 1)][r + HW][l + HW];
             {
                 CellC<T> cc;
 #pragma unroll
@@ -373,7 +401,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
                 if (PPM && i0 >= 2 && i0 <= L - 1) {
                     T m2[5];
                     load5(cu, fs, cj + (long long)(i0 - 2) * g.pi, m2);
-                    ppm_x(cc, m2, Um, Un, s.U[(i0 + 2) & (NS - 1)][r + HW][l + HW], hin, lo);
+                    ppm_x(cc, m2, Um, Un, s.U[SM::slot(i0 + 2)][r + HW][l + HW], hin, lo);
                 } else {
                     recon_x(cc, Un, Um, hin, lo);
                 }
@@ -409,12 +437,18 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     for (int i = i0; i <= i1; i++) {
         const int sm1 = (i + 2) % 3, s0 = i % 3, sp1 = (i + 1) % 3;
         const int u0 = i & 1, u1 = (i + 1) & 1;                   // Dv ring
-        const int q0 = i & (NS - 1), q1 = (i + 1) & (NS - 1);     // state ring: planes i, i+1
+        const int q0 = SM::slot(i), q1 = SM::slot(i + 1);         // state ring: planes i, i+1
         // (a) issue plane i+2 (PPM: i+3) loads (the velocities of plane i+1
         // were formed at the end of the previous iteration, or in the prologue)
-        plane_issue<T, TJE, PPM>(g, cu, i + (PPM ? 3 : 2), r, l, j, k, live, pl);
+        plane_issue<T, TJE, PPM>(s, g, cu, i + (PPM ? 3 : 2), r, l, j, k, live, pl);
         if (inter) {
             const long long c = FSL_CELL(cj + (long long)i * g.pi, fs);
+            // FP64 takes the combination's stage state from the ring and U^n at
+            // its end, from L2 where it is asked for here
+            if (sizeof(T) == 8 && a.stage != 1) {
+#pragma unroll
+                for (int q = 0; q < 5; q++) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.un + q * fs + c));
+            }
             // FP32 bulk keeps only a converted copy of the state in shared
             // memory; the FP64 operands of the combination are fetched here
             if (sizeof(T) != 8) {
@@ -525,6 +559,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
         T Fx[5], hin[5];
 #pragma unroll
         for (int q = 0; q < 5; q++) Fx[q] = hin[q] = T(0.);
+        if constexpr (SM::ASYNC) copies_done(); // the next plane's own cell
         if (inter) {
             T lo[5];
             if (i + 1 <= L) {
@@ -532,12 +567,13 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
                 ring_consts<T, TJE, PPM>(s, s.U[q1][r + HW][l + HW], i + 1, r, l, cc);
                 if constexpr (PPM) {
                     // planes i-1 .. i+2 from the ring (own column), i+3 in flight
-                    const T *Um1 = s.U[(i - 1) & (NS - 1)][r + HW][l + HW], *U0 = s.U[q0][r + HW][l + HW];
-                    const T *Up2 = s.U[(i + 2) & (NS - 1)][r + HW][l + HW];
+                    const T *Um1 = s.U[SM::slot(i - 1)][r + HW][l + HW], *U0 = s.U[q0][r + HW][l + HW];
+                    const T *Up2 = s.U[SM::slot(i + 2)][r + HW][l + HW];
                     if (i + 1 <= L - 1) {
                         T p2[5];
 #pragma unroll
-                        for (int q = 0; q < 5; q++) p2[q] = T(pl.own[q]);
+                        for (int q = 0; q < 5; q++)
+                            p2[q] = SM::ASYNC ? s.U[SM::slot(i + 3)][r + HW][l + HW][q] : T(pl.own[q]);
                         ppm_x(cc, Um1, U0, Up2, p2, hin, lo);
                     } else {
                         recon_x(cc, Up2, U0, hin, lo);
@@ -545,7 +581,8 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
                 } else {
                     T fw2[5];
 #pragma unroll
-                    for (int q = 0; q < 5; q++) fw2[q] = T(pl.own[q]);
+                    for (int q = 0; q < 5; q++)
+                        fw2[q] = SM::ASYNC ? s.U[SM::slot(i + 2)][r + HW][l + HW][q] : T(pl.own[q]);
                     recon_x(cc, fw2, s.U[q0][r + HW][l + HW], hin, lo);
                 }
             } else {
@@ -606,7 +643,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
         // planes i-1 (reciprocal ring) and i (division planes), read next
         // after the next iteration's barrier; advance the march
         if constexpr (PPM)
-            plane_store<T, TJE, PPM>(s, (i + 3) & (NS - 1), r, l, j, k, H, D, live && i + 3 <= L + 1, pl);
+            plane_store<T, TJE, PPM>(s, SM::slot(i + 3), r, l, j, k, H, D, live && i + 3 <= L + 1, pl);
         else
             plane_store<T, TJE, PPM>(s, q0, r, l, j, k, H, D, live && i + 2 <= L + 1, pl);
         if (live && i < i1) plane_prims<T, TJE, PPM, SST>(s, i + 2, r, l, mu2, mu1);

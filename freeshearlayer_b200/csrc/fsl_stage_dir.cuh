@@ -75,46 +75,51 @@ __device__ __forceinline__ double nat3(int d, double n, double a, double b)
     return a + p + q;
 }
 
-// the face states of one side (src/fluxes.c:61-83) in the frame
-__device__ __forceinline__ void face_side(int d, const double *S, double &n, double &a, double &b, double &P, double &C,
-                                          double &jo, double &jp, double &jm)
+// stage::riemann in the frame (src/fluxes.c:61-113)
+struct FaceState {
+    double Rho, P, vn, va, vb;
+};
+__device__ __noinline__ FaceState face_by_division(int d, double l0, double l1, double l2, double l3, double l4,
+                                                   double r0, double r1, double r2, double r3, double r4)
 {
-    typedef Kc<double> k;
-    const double R = S[0];
-    n = S[1] / R;
-    a = S[2] / R;
-    b = S[3] / R;
-    P = (S[4] - 0.5 * R * nat3(d, n * n, a * a, b * b)) * k::K_1;
-    C = sqrt(k::K * P / R);
-    jo = k::NK_1 * P;
-    const double RU = P / (R * C);
-    jp = n + RU;
-    jm = n - RU;
+    // the frame's components in natural order: n a b, a n b, a b n
+    const double L[5] = {l0, d == 0 ? l1 : l2, d == 0 ? l2 : d == 1 ? l1 : l3, d == 2 ? l1 : l3, l4};
+    const double R[5] = {r0, d == 0 ? r1 : r2, d == 0 ? r2 : d == 1 ? r1 : r3, d == 2 ? r1 : r3, r4};
+    FaceState o;
+    double v[3];
+    if (d == 0) {
+        riemann_div<double, 1>(L, R, o.Rho, o.P, v);
+        o.vn = v[0]; o.va = v[1]; o.vb = v[2];
+    } else if (d == 1) {
+        riemann_div<double, 2>(L, R, o.Rho, o.P, v);
+        o.vn = v[1]; o.va = v[0]; o.vb = v[2];
+    } else {
+        riemann_div<double, 3>(L, R, o.Rho, o.P, v);
+        o.vn = v[2]; o.va = v[0]; o.vb = v[1];
+    }
+    return o;
 }
 
-// stage::riemann in the frame (src/fluxes.c:85-113)
 __device__ __forceinline__ void face_riemann(int d, const double *Lm, const double *Rp, double &Rho, double &P,
                                              double &vn, double &va, double &vb)
 {
     typedef Kc<double> k;
-    double ln, la, lb, lP, lC, ljo, ljp, ljm, rn, ra, rb, rP, rC, rjo, rjp, rjm;
-    face_side(d, Lm, ln, la, lb, lP, lC, ljo, ljp, ljm);
-    face_side(d, Rp, rn, ra, rb, rP, rC, rjo, rjp, rjm);
-    const double Un = 0.5 * (ln + rn), C = 0.5 * (lC + rC);
-    const bool pp = Un + C > 0., pm = Un - C > 0., po = Un > 0.;
-    const double al_p = k::K_1_2 * (pp ? (ljm - ljp) : (rjm - rjp)) / (pp ? ljo : rjo);
-    const double Jp = pp ? ljp : rjp;
-    const double al_m = k::K_1_2 * (pm ? (ljp - ljm) : (rjp - rjm)) / (pm ? ljo : rjo);
-    const double Jm = pm ? ljm : rjm;
-    double al_o = k::K05 * (po ? (ljp - ljm) : (rjp - rjm));
-    al_o = -al_o * al_o;
-    const double Jo = po ? ljo : rjo;
-    P = (Jp - Jm) / (al_p - al_m);
-    vn = Jp - al_p * P;
-    Rho = (Jo - P) / al_o;
-    const bool up = vn > 0;
+    double ln, la, lb, ly, lC, lRU, rn, ra, rb, ry, rC, rRU;
+    bool ok = riemann_side64(Lm[0], Lm[1], Lm[2], Lm[3], ln, la, lb, ly);
+    ok = riemann_side64(Rp[0], Rp[1], Rp[2], Rp[3], rn, ra, rb, ry) && ok;
+    const double lP = (Lm[4] - 0.5 * Lm[0] * nat3(d, ln * ln, la * la, lb * lb)) * k::K_1;
+    const double rP = (Rp[4] - 0.5 * Rp[0] * nat3(d, rn * rn, ra * ra, rb * rb)) * k::K_1;
+    ok = riemann_side64(Lm[0], lP, ly, lC, lRU) && ok;
+    ok = riemann_side64(Rp[0], rP, ry, rC, rRU) && ok;
+    ok = riemann_mid64(ln, lP, lC, lRU, rn, rP, rC, rRU, Rho, P, vn) && ok;
+    const bool up = vn > 0.;
     va = up ? la : ra;
     vb = up ? lb : rb;
+    if (!ok) {
+        const FaceState o = face_by_division(d, Lm[0], Lm[1], Lm[2], Lm[3], Lm[4], Rp[0], Rp[1], Rp[2], Rp[3], Rp[4]);
+        Rho = o.Rho; P = o.P;
+        vn = o.vn; va = o.va; vb = o.vb;
+    }
 }
 
 template <bool SST>
@@ -211,14 +216,13 @@ __global__ void __launch_bounds__(NT, 1) k_stage_dir(DirArgs A)
             const double *u = U0 + (p & 3) * UP + pr * UR + pc * 5;
 #pragma unroll
             for (int q = 0; q < 5; q++) c.u[q] = u[q];
-            cell_roots(c);
+            double dv[4];
+            cell_prims64(c, dv);
             double *v = R0 + ((p + 3) % 3) * RP + pr * RR + pc * 3, *o = V0 + (p & 1) * VP + pr * VR + pc * 5,
                    *w = K0 + (p & 1) * KP + pr * KR + pc * 4;
             v[0] = c.U; v[1] = c.V; v[2] = c.W;
             w[0] = c.C; w[1] = c.ll; w[2] = c.ee;
             w[3] = c.U * c.U + c.V * c.V + c.W * c.W;
-            double dv[4];
-            vdiv(c.u, dv);
             o[0] = dv[0]; o[1] = dv[1]; o[2] = dv[2]; o[3] = dv[3];
             if constexpr (!SST) o[4] = 0.5 * (mu_next + mu_prev);
         };
