@@ -583,6 +583,18 @@ static double *stage_state(Ctx &c)
     return c.stage_next == 2 ? c.Up : c.stage_next == 3 ? c.Uq : c.U;
 }
 
+// Memory of the context's own device that a kernel can read and write in place
+// (other buffers go through the scratch buffer and a copy).
+static bool on_device(const Ctx &c, const double *buf)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, buf) != cudaSuccess) {
+        cudaGetLastError(); // an unregistered host pointer on some drivers
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == c.device && (uintptr_t)buf % sizeof(double) == 0;
+}
+
 // gather planes i0.. of the current stage state into buf, queued on the
 // context's stream (the one scratch buffer is reused in stream order)
 static int get_planes_q(fsl_ctx *h, int i0, int n, double *buf)
@@ -592,9 +604,10 @@ static int get_planes_q(fsl_ctx *h, int i0, int n, double *buf)
     Ctx &c = h->c;
     if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_get_planes: the current-stage buffer is not U^n");
     const size_t bytes = (size_t)n * c.p.HIG * 5 * c.p.DEP * sizeof(double);
-    launch_state_gather(c, stage_state(c), c.stage_dev, i0, n);
+    const bool direct = on_device(c, buf);
+    launch_state_gather(c, stage_state(c), direct ? buf : c.stage_dev, i0, n);
     CKL();
-    if (bytes) CK(cudaMemcpyAsync(buf, c.stage_dev, bytes, cudaMemcpyDefault, c.stream));
+    if (bytes && !direct) CK(cudaMemcpyAsync(buf, c.stage_dev, bytes, cudaMemcpyDefault, c.stream));
     return FSL_OK;
 }
 
@@ -607,8 +620,9 @@ static int set_planes_q(fsl_ctx *h, int i0, int n, const double *buf)
     const size_t bytes = (size_t)n * c.p.HIG * 5 * c.p.DEP * sizeof(double);
     // planes outside the Courant range leave the owned maximum as it is
     if (c.stage_next == 0 && n > 0 && i0 <= c.co_i1 && i0 + n - 1 >= c.co_i0) c.co_valid = false;
-    if (bytes) CK(cudaMemcpyAsync(c.stage_dev, buf, bytes, cudaMemcpyDefault, c.stream));
-    launch_state_scatter(c, stage_state(c), c.stage_dev, i0, n);
+    const bool direct = on_device(c, buf);
+    if (bytes && !direct) CK(cudaMemcpyAsync(c.stage_dev, buf, bytes, cudaMemcpyDefault, c.stream));
+    launch_state_scatter(c, stage_state(c), direct ? buf : c.stage_dev, i0, n);
     CKL();
     return FSL_OK;
 }
@@ -1276,7 +1290,7 @@ int fsl_plane_sums(fsl_ctx *h, double *rows)
 {
     if (!h || !rows) return FSL_ERR_ARG;
     Ctx &c = h->c;
-    double *d = c.stage_dev; // scratch: 8*HIG <= LEN*HIG*5*DEP
+    double *d = c.stage_dev; // scratch: 8 HIG (1 + LEN / 2) <= LEN HIG 5 DEP
     launch_plane_sums(c, c.U, c.co_i0, c.co_i1 - c.co_i0 + 1, d);
     CKL();
     CK(cudaMemcpyAsync(rows, d, 8 * (size_t)c.p.HIG * sizeof(double), cudaMemcpyDeviceToHost, c.stream));

@@ -512,32 +512,35 @@ __global__ void k_judge_rows(Grid g, const TA *__restrict__ a, const TB *__restr
 // ---------------------------------------------------------------------------
 // state transfer and diagnostics
 // ---------------------------------------------------------------------------
-__global__ void k_state_scatter(Grid g, double *__restrict__ dst, const double *__restrict__ packed, int i0, int ni)
+// Planes i0 .. i0+ni-1 (1-based interior planes) between the padded fields and
+// the state layout, one warp per row of DEP values, four loads in flight per
+// lane, pairs of values where every packed row starts on 16 bytes.  Bound by
+// memory: 512x256x256 928 us -> 430 us a direction (three 64-bit divisions per
+// value before).
+template <bool GATHER, typename V>
+__global__ void __launch_bounds__(256) k_state_rows(Grid g, double *__restrict__ fields, double *__restrict__ packed,
+                                                    int i0, unsigned nrows)
 {
-    const long long n = (long long)ni * g.H * 5 * g.D;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % g.D);
-        long long r = t / g.D;
-        const int v = (int)(r % 5); r /= 5;
-        const int j = (int)(r % g.H);
-        const int i = (int)(r / g.H);
-        dst[v * g.fstride + FSL_CELL(g.idx(i + i0, j + 1, k + 1), g.fstride)] = packed[t];
-    }
-}
-
-// planes i0 .. i0+ni-1 (1-based interior planes) in the state layout
-__global__ void k_state_gather(Grid g, const double *__restrict__ src, double *__restrict__ packed, int i0, int ni)
-{
-    const long long n = (long long)ni * g.H * 5 * g.D;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % g.D);
-        long long r = t / g.D;
-        const int v = (int)(r % 5); r /= 5;
-        const int j = (int)(r % g.H);
-        const int i = (int)(r / g.H);
-        packed[t] = src[v * g.fstride + FSL_CELL(g.idx(i + i0, j + 1, k + 1), g.fstride)];
+    constexpr int W = sizeof(V) / sizeof(double), UN = 4;
+    const unsigned H = (unsigned)g.H, n = (unsigned)g.D / W, l = threadIdx.x & 31;
+    for (unsigned row = blockIdx.x * 8u + (threadIdx.x >> 5); row < nrows; row += gridDim.x * 8u) {
+        const unsigned ij = row / 5u, v = row - ij * 5u, ii = ij / H, j = ij - ii * H;
+        const long long c = g.idx((int)ii + i0, (int)j + 1, 1);
+        (void)FSL_CELL(c, g.fstride);
+        (void)FSL_CELL(c + g.D - 1, g.fstride);
+        V *f = reinterpret_cast<V *>(fields + v * g.fstride + c);
+        V *p = reinterpret_cast<V *>(packed + (long long)row * g.D);
+        const V *src = GATHER ? f : p;
+        V *dst = GATHER ? p : f;
+        for (unsigned k = l; k < n; k += 32 * UN) {
+            V x[UN];
+#pragma unroll
+            for (int q = 0; q < UN; q++)
+                if (k + 32 * q < n) x[q] = src[k + 32 * q];
+#pragma unroll
+            for (int q = 0; q < UN; q++)
+                if (k + 32 * q < n) dst[k + 32 * q] = x[q];
+        }
     }
 }
 
@@ -583,24 +586,27 @@ __global__ void k_sums_final(const double *__restrict__ partials, int np, double
     }
 }
 
-// One block per y row: sums over the x-z plane (interior planes i0 ..
-// i0+ni-1) of rho, rho u, rho v, rho w, rho uu, rho vv, rho ww, rho uv.
-__global__ void k_plane_sums(Grid g, int i0, int ni, const double *__restrict__ U, double *__restrict__ rows)
+// Block (y row, segment of the planes i0 .. i0+ni-1): sums over its cells of
+// rho, rho u, rho v, rho w, rho uu, rho vv, rho ww, rho uv; a warp per plane.
+__global__ void __launch_bounds__(256) k_plane_sums(Grid g, int i0, int ni, int seg, const double *__restrict__ U,
+                                                    double *__restrict__ parts)
 {
-    const int j = blockIdx.x + 1;
-    const long long n = (long long)ni * g.D;
+    const int j = blockIdx.x + 1, w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int ib = (int)blockIdx.y * seg, ie = min(ni, ib + seg);
+    const long long fs = g.fstride;
     double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = (int)(t % g.D) + 1;
-        const int i = (int)(t / g.D) + i0;
-        const long long c = FSL_CELL(g.idx(i, j, k), g.fstride);
-        const double r = U[c], u = U[g.fstride + c] / r, v = U[2 * g.fstride + c] / r,
-                     w = U[3 * g.fstride + c] / r;
-        s[0] += r; s[1] += r * u; s[2] += r * v; s[3] += r * w;
-        s[4] += r * u * u; s[5] += r * v * v; s[6] += r * w * w; s[7] += r * u * v;
+    for (int i = ib + w; i < ie; i += 8) {
+        const long long c0 = g.idx(i + i0, j, 1);
+#pragma unroll 2
+        for (int k = l; k < g.D; k += 32) {
+            const long long c = FSL_CELL(c0 + k, fs);
+            const double r = U[c], m1 = U[fs + c], m2 = U[2 * fs + c], m3 = U[3 * fs + c];
+            const double u = m1 / r, v = m2 / r, ww = m3 / r;
+            s[0] += r; s[1] += r * u; s[2] += r * v; s[3] += r * ww;
+            s[4] += r * u * u; s[5] += r * v * v; s[6] += r * ww * ww; s[7] += r * u * v;
+        }
     }
-    __shared__ double sm[8][32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    __shared__ double sm[8][8];
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         double x = s[q];
@@ -611,9 +617,20 @@ __global__ void k_plane_sums(Grid g, int i0, int ni, const double *__restrict__ 
     __syncthreads();
     if (threadIdx.x < 8) {
         double x = 0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) x += sm[threadIdx.x][q];
-        rows[(long long)blockIdx.x * 8 + threadIdx.x] = x;
+#pragma unroll
+        for (int q = 0; q < 8; q++) x += sm[threadIdx.x][q];
+        parts[((long long)blockIdx.y * g.H + blockIdx.x) * 8 + threadIdx.x] = x;
     }
+}
+
+// the segments' sums of every row, in order
+__global__ void k_plane_sums_final(int n, int nseg, const double *__restrict__ parts, double *__restrict__ rows)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    double x = 0;
+    for (int q = 0; q < nseg; q++) x += parts[(long long)q * n + t];
+    rows[t] = x;
 }
 
 inline dim3 cells_grid(const Grid &g, dim3 b, int ni, int nj, int nk)
@@ -706,20 +723,27 @@ void launch_courant_apply(Ctx &c)
     prof_end(c, FSL_K_CFL, 1);
 }
 
-void launch_state_scatter(Ctx &c, double *dst, const double *packed, int i0, int ni)
+template <bool GATHER> static void state_rows(Ctx &c, double *fields, double *packed, int i0, int ni)
 {
     if (ni <= 0) return;
+    const Grid &g = c.g;
+    const unsigned nrows = (unsigned)((long long)ni * g.H * 5); // at most 2^31 cells of DEP >= 2
+    const unsigned nblk = std::min((nrows + 7u) / 8u, 148u * 8u);
     prof_begin(c, FSL_K_OTHER);
-    k_state_scatter<<<148 * 8, 256, 0, c.stream>>>(c.g, dst, packed, i0, ni);
+    if (g.D % 2 == 0 && (uintptr_t)packed % 16 == 0)
+        k_state_rows<GATHER, double2><<<nblk, 256, 0, c.stream>>>(g, fields, packed, i0, nrows);
+    else k_state_rows<GATHER, double><<<nblk, 256, 0, c.stream>>>(g, fields, packed, i0, nrows);
     prof_end(c, FSL_K_OTHER, 1);
+}
+
+void launch_state_scatter(Ctx &c, double *dst, const double *packed, int i0, int ni)
+{
+    state_rows<false>(c, dst, const_cast<double *>(packed), i0, ni);
 }
 
 void launch_state_gather(Ctx &c, const double *src, double *packed, int i0, int ni)
 {
-    if (ni <= 0) return;
-    prof_begin(c, FSL_K_OTHER);
-    k_state_gather<<<148 * 8, 256, 0, c.stream>>>(c.g, src, packed, i0, ni);
-    prof_end(c, FSL_K_OTHER, 1);
+    state_rows<true>(c, const_cast<double *>(src), packed, i0, ni);
 }
 
 void launch_sums(Ctx &c, const double *U, int i0, int ni, double *out5)
@@ -742,11 +766,18 @@ void launch_judge_rows(Ctx &c, const float *a, const float *b, double *rows) { j
 void launch_judge_rows(Ctx &c, const float *a, const double *b, double *rows) { judge_rows_t(c, a, b, rows); }
 void launch_judge_rows(Ctx &c, const double *a, const double *b, double *rows) { judge_rows_t(c, a, b, rows); }
 
+// rows: 8 HIG doubles, followed by scratch for the segments (8 HIG doubles each,
+// at most LEN / 2 of them).  One block per row left most SMs a single block's
+// latency: 512x256x256 871 -> 250 us.
 void launch_plane_sums(Ctx &c, const double *U, int i0, int ni, double *rows)
 {
+    const int H = c.g.H;
+    const int want = std::max(1, std::min((8 * c.sms + H - 1) / H, ni / 2)); // eight blocks an SM
+    const int seg = (ni + want - 1) / want, nseg = (ni + seg - 1) / seg;
     prof_begin(c, FSL_K_OTHER);
-    k_plane_sums<<<c.g.H, 256, 0, c.stream>>>(c.g, i0, ni, U, rows);
-    prof_end(c, FSL_K_OTHER, 1);
+    k_plane_sums<<<dim3(H, nseg), 256, 0, c.stream>>>(c.g, i0, ni, seg, U, rows + 8 * (size_t)H);
+    k_plane_sums_final<<<(8 * H + 127) / 128, 128, 0, c.stream>>>(8 * H, nseg, rows + 8 * (size_t)H, rows);
+    prof_end(c, FSL_K_OTHER, 2);
 }
 
 } // namespace fsl
