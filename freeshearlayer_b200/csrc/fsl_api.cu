@@ -949,8 +949,8 @@ int step_prelude32(Ctx &c)
     else launch_courant(c);
     c.step++;
     draw(c);
-    launch_ghost(c, c.U);
-    if (!forms_boundaries(c)) launch_bface32(c, c.U, c.dist);
+    if (forms_boundaries(c)) launch_ghost(c, c.U);
+    else launch_boundary32(c, c.U, c.dist);
     return step_sgs(c);
 }
 } // namespace fsl
@@ -1016,16 +1016,16 @@ int fsl_step_phased(fsl_ctx *h, int nsteps)
     return FSL_OK;
 }
 
-// boundary outer states of the fused stage kernels, in the path's precision
-static void launch_faces(Ctx &c, const double *cur)
+// the boundary pass before a fused stage, in the path's precision
+static void launch_boundaries(Ctx &c, double *cur)
 {
-    if (c.p.precision == FSL_PREC_FP32) launch_bface32(c, cur, c.dist);
-    else launch_bface(c, cur, c.dist);
+    if (c.p.precision == FSL_PREC_FP32) launch_boundary32(c, cur, c.dist);
+    else launch_boundary(c, cur, c.dist);
 }
 
-// Fused path: per stage a ghost fill, the boundary outer states and one
-// fused stage kernel (kernels that form the boundaries themselves need
-// neither pass between stages); stages ping-pong U^n -> Up -> Uq -> U^n.
+// Fused path: per stage the boundary pass and one fused stage kernel (kernels
+// that form the boundaries themselves need no pass between stages); stages
+// ping-pong U^n -> Up -> Uq -> U^n.
 int fsl_step(fsl_ctx *h, int nsteps)
 {
     ApiRange range_("fsl_step");
@@ -1054,8 +1054,8 @@ int fsl_step(fsl_ctx *h, int nsteps)
         draw(c);
         // U^n's ghost layer: the previous step's last FP32-bulk stage wrote it,
         // unless that step ran before this call
-        if (!(fb && fp32) || n == 0) launch_ghost(c, c.U);
-        if (!fb) launch_faces(c, c.U);
+        if (!fb) launch_boundaries(c, c.U);
+        else if (!fp32 || n == 0) launch_ghost(c, c.U);
         c.vel_fresh = vel && n > 0;
         rc = step_sgs(c);
         c.vel_fresh = false;
@@ -1063,10 +1063,7 @@ int fsl_step(fsl_ctx *h, int nsteps)
         double *const state[4] = {c.U, c.Up, c.Uq, c.U};
         for (int s = 1; s <= 3; s++) {
             double *in = state[s - 1], *out = state[s];
-            if (s > 1 && !fb) {
-                launch_ghost(c, in);
-                launch_faces(c, in);
-            }
+            if (s > 1 && !fb) launch_boundaries(c, in);
             const int e = fp32 ? launch_stage32(c, s, in, c.U, out, s == 3, s == 3 ? vel : nullptr)
                                : launch_stage(c, s, in, c.U, out, s == 3);
             if (e) return fail(c, FSL_ERR_CUDA, "stage kernel");
@@ -1098,32 +1095,26 @@ int fsl_step_stage(fsl_ctx *h)
         else launch_courant(c);
         c.step++;
         draw(c);
-        launch_ghost(c, c.U);
-        if (fp32) launch_bface32(c, c.U, c.dist);
-        else launch_bface(c, c.U, c.dist);
+        launch_boundaries(c, c.U);
         if ((rc = step_sgs(c))) return rc;
         const int e = fp32 ? launch_stage32(c, 1, c.U, c.U, c.Up) : launch_stage(c, 1, c.U, c.U, c.Up);
         if (e) return fail(c, FSL_ERR_CUDA, "stage kernel");
         c.stage_next = 2;
     } else if (c.stage_next == 2) {
         if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step_stage: the current-stage buffer is not U^n");
-        launch_ghost(c, c.Up);
+        launch_boundaries(c, c.Up);
         if (fp32) {
-            launch_bface32(c, c.Up, c.dist);
             launch_stage32(c, 2, c.Up, c.U, c.Uq);
         } else {
-            launch_bface(c, c.Up, c.dist);
             launch_stage(c, 2, c.Up, c.U, c.Uq);
         }
         c.stage_next = 3;
     } else {
         if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step_stage: the current-stage buffer is not U^n");
-        launch_ghost(c, c.Uq);
+        launch_boundaries(c, c.Uq);
         if (fp32) {
-            launch_bface32(c, c.Uq, c.dist);
             launch_stage32(c, 3, c.Uq, c.U, c.U, true);
         } else {
-            launch_bface(c, c.Uq, c.dist);
             launch_stage(c, 3, c.Uq, c.U, c.U, true);
         }
         c.co_valid = true;

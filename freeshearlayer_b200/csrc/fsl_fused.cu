@@ -16,9 +16,9 @@ static stage::BF<double> bf64(Ctx &c)
     return b;
 }
 
-void launch_bface(Ctx &c, const double *cur, const Disturb &d)
+void launch_boundary(Ctx &c, double *cur, const Disturb &d)
 {
-    stage::launch_bface_t<double>(c, cur, d, bf64(c));
+    stage::launch_boundary_t<double>(c, cur, d, bf64(c));
 }
 
 // How a domain's tiles (tj x tk output cells) are cut along x when one block

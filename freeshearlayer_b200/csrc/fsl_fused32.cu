@@ -24,9 +24,9 @@ static stage::BF<float> bf32(Ctx &c)
     return b;
 }
 
-void launch_bface32(Ctx &c, const double *cur, const Disturb &d)
+void launch_boundary32(Ctx &c, double *cur, const Disturb &d)
 {
-    stage::launch_bface_t<float>(c, cur, d, bf32(c));
+    stage::launch_boundary_t<float>(c, cur, d, bf32(c));
 }
 
 template <bool SST>

@@ -221,13 +221,14 @@ void launch_sums(Ctx &c, const double *U, int i0, int ni, double *out5);
 void launch_plane_sums(Ctx &c, const double *U, int i0, int ni, double *rows);
 
 // ---- fused path (fsl_fused.cu) ----------------------------------------------
-void launch_bface(Ctx &c, const double *cur, const Disturb &d);
+// ghost layer of cur and the outer states of the boundary faces
+void launch_boundary(Ctx &c, double *cur, const Disturb &d);
 // One RK3 stage: cur (ghosts filled) -> out; un = U^n.
 int launch_stage(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant = false);
 // whether launch_stage runs the direction-split kernel (rows 0, small grids)
 bool stage_splits_directions(const Ctx &c);
 // FP32-bulk variants (fsl_fused32.cu): boundary states in bf32, SGS viscosity in mu32.
-void launch_bface32(Ctx &c, const double *cur, const Disturb &d);
+void launch_boundary32(Ctx &c, double *cur, const Disturb &d);
 // vel (full-lane tile, temporal setup, stage 3 only): also write the FP32
 // velocities of `out` into that field (the closure's feature velocities)
 int launch_stage32(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant = false,

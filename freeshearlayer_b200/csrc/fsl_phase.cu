@@ -12,6 +12,7 @@
 #include "fsl_dyn.cuh"
 #include "fsl_internal.h"
 #include "fsl_phys.cuh"
+#include "fsl_stage.cuh"
 
 FSL_CHK_EXPORT(phase)
 
@@ -33,72 +34,12 @@ __device__ __forceinline__ long long izf(int L, int H, int D, int i, int j, int 
 }
 
 // ---------------------------------------------------------------------------
-// A1 ghost cells (src/boundCondInGhostCells.c:10-96).  The reference fills x,
-// then z over all i, then y over all i and k; every ghost value is therefore a
-// composition of copies of one interior cell (or of the inflow profile).  Each
-// thread evaluates that composition for one ghost cell, so all ghost cells are
-// written in one pass with the reference's values, edges and corners included.
+// A1 ghost cells (src/boundCondInGhostCells.c:10-96), one thread per cell.
 // ---------------------------------------------------------------------------
 __global__ void k_ghost(Grid g, int setup, double *__restrict__ u)
 {
-    const int L = g.L, H = g.H, D = g.D;
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nx = 2LL * (H + 2) * (D + 2), ny = 2LL * L * (D + 2), nz = 2LL * L * H;
-    int i, j, k;
-    if (t < nx) {
-        long long a = (long long)(H + 2) * (D + 2);
-        i = (t / a) ? L + 1 : 0;
-        long long r = t % a;
-        j = (int)(r / (D + 2));
-        k = (int)(r % (D + 2));
-    } else if ((t -= nx) < ny) {
-        long long a = (long long)L * (D + 2);
-        j = (t / a) ? H + 1 : 0;
-        long long r = t % a;
-        i = 1 + (int)(r / (D + 2));
-        k = (int)(r % (D + 2));
-    } else if ((t -= ny) < nz) {
-        long long a = (long long)L * H;
-        k = (t / a) ? D + 1 : 0;
-        long long r = t % a;
-        i = 1 + (int)(r / H);
-        j = 1 + (int)(r % H);
-    } else {
-        return;
-    }
-    const bool spatial = (setup == FSL_SETUP_SPATIAL);
-    bool flip = false;
-    int jj = j, kk = k;
-    if (j == 0) { jj = 1; flip = spatial; }
-    else if (j == H + 1) { jj = H; flip = spatial; }
-    if (k == 0) kk = D;
-    else if (k == D + 1) kk = 1;
-    double v[5];
-    const long long fs = g.fstride;
-    typedef Kc<double> kc;
-    if (i == 0 && spatial) {
-        // inflow step profile, :17-40
-        const double P = 100000., R = 1.0;
-        const double U = (jj <= H / 2) ? 76.4 : 200;
-        v[0] = R; v[1] = R * U; v[2] = 0.; v[3] = 0.;
-        v[4] = P / kc::K_1 + 0.5 * R * (U * U);
-    } else {
-        int si = i;
-        if (i == 0) si = L;               // temporal: periodic x
-        else if (i == L + 1) si = spatial ? L : 1;
-        long long s = FSL_CELL(g.idx(si, jj, kk), fs);
-#pragma unroll
-        for (int q = 0; q < 5; q++) v[q] = u[q * fs + s];
-        if (i == L + 1 && spatial) {
-            // outflow, :44-52: momenta copied, E rebuilt at P = 1e5
-            const double P = 100000.;
-            v[4] = P / kc::K_1 + 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) / v[0];
-        }
-    }
-    if (flip) v[2] = -v[2];
-    long long d = FSL_CELL(g.idx(i, j, k), fs);
-#pragma unroll
-    for (int q = 0; q < 5; q++) u[q * fs + d] = v[q];
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < stage::ghost_cells(g)) stage::ghost_cell(g, setup == FSL_SETUP_SPATIAL, u, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -645,7 +586,7 @@ inline dim3 cells_grid(const Grid &g, dim3 b, int ni, int nj, int nk)
 void launch_ghost(Ctx &c, double *cur)
 {
     const Grid &g = c.g;
-    const long long n = 2LL * (g.H + 2) * (g.D + 2) + 2LL * g.L * (g.D + 2) + 2LL * g.L * g.H;
+    const long long n = stage::ghost_cells(g);
     prof_begin(c, FSL_K_BC);
     k_ghost<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(g, c.k.setup, cur);
     prof_end(c, FSL_K_BC, 1);

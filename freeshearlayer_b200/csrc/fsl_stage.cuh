@@ -16,7 +16,7 @@
 // stage result written once.  Plane i+2 is fetched into registers at the top
 // of iteration i and stored to shared memory at its end, hiding the load
 // latency behind the flux work.  Domain-boundary faces take their outer state
-// from the boundary pass (k_bface), which applies the reference's interface
+// from the boundary pass (k_boundary), which applies the reference's interface
 // rules (src/bounCondOnInterfaces.c:11-110) to the reconstructed boundary cells.
 #pragma once
 
@@ -77,24 +77,121 @@ __device__ __forceinline__ void ppm_at_x(const Grid &g, const double *__restrict
     ppm_x(cc, m2, m1, p1, p2, hi, lo);
 }
 
-// Outer states of one domain-boundary face (src/bounCondOnInterfaces.c:11-110):
-// face t of the x (HIG DEP), y (LEN DEP) and z (LEN HIG) boundary lists.
-// Not inlined: the boundary pass and the persistent multi-domain stage
-// kernel run this one compiled body, so their FP32 results agree bit for bit.
-template <typename T>
-__device__ __noinline__ void bface_one(Grid g, int setup, int BL_HIG, Disturb d, const double *__restrict__ u,
-                                       BF<T> bf, long long t)
+// State on the outer face of the boundary cell c in direction DIR: the upper
+// face (UP) or the lower one, from the cell, its inner neighbour and the ghost
+// value g5 beyond the face (FP64, natural order).
+template <typename T, int DIR, bool UP>
+__device__ __forceinline__ void edge_state(const Grid &g, const double *__restrict__ u, long long c, const double *g5,
+                                           T *out)
+{
+    const long long fs = g.fstride;
+    CellC<T> cc;
+    load5(u, fs, c, cc.u);
+    cell_consts(cc);
+    const long long d = DIR == 0 ? g.pi : DIR == 1 ? (long long)g.pk : 1LL;
+    const int p1 = DIR == 0 ? 1 : DIR == 1 ? 2 : 3;
+    const int p2 = DIR == 0 ? 2 : DIR == 1 ? 3 : 1;
+    const int p3 = DIR == 0 ? 3 : DIR == 1 ? 1 : 2;
+    T in[5], go[5], other[5];
+    const long long ci = FSL_CELL(UP ? c - d : c + d, fs);
+    in[0] = T(u[ci]); in[1] = T(u[p1 * fs + ci]); in[2] = T(u[p2 * fs + ci]);
+    in[3] = T(u[p3 * fs + ci]); in[4] = T(u[4 * fs + ci]);
+    go[0] = T(g5[0]); go[1] = T(g5[p1]); go[2] = T(g5[p2]); go[3] = T(g5[p3]); go[4] = T(g5[4]);
+    T *hi = UP ? out : other, *lo = UP ? other : out;
+    const T *fw = UP ? go : in, *bw = UP ? in : go;
+    if (DIR == 0) recon_x(cc, fw, bw, hi, lo);
+    else if (DIR == 1) recon_y(cc, fw, bw, hi, lo);
+    else recon_z(cc, fw, bw, hi, lo);
+}
+
+// The ghost value beyond the interior boundary cell s in direction DIR, before
+// the other directions' copies (src/boundCondInGhostCells.c:10-96): `c` the cell
+// it copies, with the spatial setup's slip wall and outflow.  Explicitly rounded,
+// so both precisions' translation units form the ghost pass's bits.
+__device__ __forceinline__ void ghost_value(const double *__restrict__ u, long long fs, long long c, bool flip,
+                                            bool outflow, double *v)
+{
+#pragma unroll
+    for (int q = 0; q < 5; q++) v[q] = u[q * fs + c];
+    if (outflow) { // :44-52: momenta copied, E rebuilt at P = 1e5
+        const double q = __dadd_rn(__dadd_rn(__dmul_rn(v[1], v[1]), __dmul_rn(v[2], v[2])), __dmul_rn(v[3], v[3]));
+        v[4] = __dadd_rn(__ddiv_rn(100000., 0.4), __ddiv_rn(__dmul_rn(0.5, q), v[0]));
+    }
+    if (flip) v[2] = -v[2];
+}
+
+// Ghost cell t of the ghost layer (x planes, y rows and z columns in turn).  The
+// reference fills x, then z over all i, then y over all i and k; every ghost
+// value is therefore a composition of copies of one interior cell (or of the
+// inflow profile), which is evaluated here for one cell, edges and corners
+// included.  32-bit divisions: no list is longer than 2^32 on 2^31 cells.
+__device__ __forceinline__ void ghost_cell(const Grid &g, bool spatial, double *__restrict__ u, long long t)
 {
     const int L = g.L, H = g.H, D = g.D;
-    const long long nx = (long long)H * D, ny = (long long)L * D, nz = (long long)L * H;
-    const bool spatial = (setup == FSL_SETUP_SPATIAL);
+    const long long ax = (long long)(H + 2) * (D + 2), ay = (long long)L * (D + 2), az = (long long)L * H;
+    int i, j, k;
+    if (t < 2 * ax) {
+        const bool up = t >= ax;
+        const unsigned r = (unsigned)(up ? t - ax : t), w = (unsigned)D + 2u;
+        i = up ? L + 1 : 0;
+        j = (int)(r / w);
+        k = (int)(r - (unsigned)j * w);
+    } else if ((t -= 2 * ax) < 2 * ay) {
+        const bool up = t >= ay;
+        const unsigned r = (unsigned)(up ? t - ay : t), w = (unsigned)D + 2u, q = r / w;
+        j = up ? H + 1 : 0;
+        i = 1 + (int)q;
+        k = (int)(r - q * w);
+    } else {
+        t -= 2 * ay;
+        const bool up = t >= az;
+        const unsigned r = (unsigned)(up ? t - az : t), w = (unsigned)H, q = r / w;
+        k = up ? D + 1 : 0;
+        i = 1 + (int)q;
+        j = 1 + (int)(r - q * w);
+    }
+    const int jj = j == 0 ? 1 : j == H + 1 ? H : j, kk = k == 0 ? D : k == D + 1 ? 1 : k;
+    const bool flip = spatial && jj != j;
+    const long long fs = g.fstride;
+    double v[5];
+    if (i == 0 && spatial) {
+        // inflow step profile, :17-40
+        const double P = 100000., R = 1.0;
+        const double U = (jj <= H / 2) ? 76.4 : 200;
+        v[0] = R; v[1] = R * U; v[2] = 0.; v[3] = 0.;
+        v[4] = __dadd_rn(P / 0.4, __dmul_rn(0.5 * R, __dmul_rn(U, U)));
+        if (flip) v[2] = -v[2];
+    } else {
+        const int si = i == 0 ? L : i == L + 1 ? (spatial ? L : 1) : i;
+        ghost_value(u, fs, FSL_CELL(g.idx(si, jj, kk), fs), flip, spatial && i == L + 1, v);
+    }
+    const long long d = FSL_CELL(g.idx(i, j, k), fs);
+#pragma unroll
+    for (int q = 0; q < 5; q++) u[q * fs + d] = v[q];
+}
+__host__ __device__ inline long long ghost_cells(const Grid &g)
+{
+    return 2LL * (g.H + 2) * (g.D + 2) + 2LL * g.L * (g.D + 2) + 2LL * g.L * g.H;
+}
+
+// Outer states of one domain-boundary face (src/bounCondOnInterfaces.c:11-110):
+// face t of the x (HIG DEP), y (LEN DEP) and z (LEN HIG) boundary lists, the lower
+// boundary's face or (upper) the other's.
+template <typename T>
+__device__ __forceinline__ void bface_one(const Grid &g, bool spatial, int BL_HIG, const Disturb &d,
+                                          const double *__restrict__ u, const BF<T> &bf, long long t, bool upper)
+{
+    const int L = g.L, H = g.H, D = g.D;
+    const long long nx = (long long)H * D, ny = (long long)L * D, nz = (long long)L * H, fs = g.fstride;
     typedef Kc<T> kc;
-    T hi[5], lo[5];
+    T o[5];
+    double gv[5];
     if (t < nx) {
-        const int jf = (int)(t / D), kf = (int)(t % D);
+        const unsigned r = (unsigned)t;
+        const int jf = (int)(r / (unsigned)D), kf = (int)(r - (unsigned)jf * (unsigned)D);
         const int j = jf + 1, k = kf + 1;
-        const long long fo = t;
-        if (spatial) {
+        const long long fo = FSL_FACE(t, nx);
+        if (spatial && !upper) {
             // inflow profile in the reference's FP64 arithmetic (:17-60)
             const double P = 100000., R = 1.0;
             double U, V = 0., W = 0., v[5];
@@ -115,47 +212,71 @@ __device__ __noinline__ void bface_one(Grid g, int setup, int BL_HIG, Disturb d,
                 v[0] = R; v[1] = R * U; v[2] = 0.; v[3] = 0.; v[4] = P / 0.4 + 0.5 * R * (U * U);
             }
 #pragma unroll
-            for (int q = 0; q < 5; q++) bf.x0[q * nx + FSL_FACE(fo, nx)] = T(v[q]);
+            for (int q = 0; q < 5; q++) bf.x0[q * nx + fo] = T(v[q]);
+        } else if (spatial) {
             // :62-71 outflow from the minus state of face LEN
-            recon_at<T, 0>(g, u, g.idx(L, j, k), hi, lo);
-            const T r = hi[0], mu_ = hi[1], mv = hi[2], mw = hi[3];
+            const long long c = g.idx(L, j, k);
+            ghost_value(u, fs, FSL_CELL(c, fs), false, true, gv);
+            edge_state<T, 0, true>(g, u, c, gv, o);
+            const T r_ = o[0], mu_ = o[1], mv = o[2], mw = o[3];
             const T P_ = T(100000.);
-            const long long fc = FSL_FACE(fo, nx);
-            bf.xL[fc] = r; bf.xL[nx + fc] = mu_; bf.xL[2 * nx + fc] = mv; bf.xL[3 * nx + fc] = mw;
-            bf.xL[4 * nx + fc] = P_ / kc::K_1 + T(0.5) * (mu_ * mu_ + mv * mv + mw * mw) / r;
-        } else { // periodic x, the reference's z rule (:94-109)
-            recon_at<T, 0>(g, u, g.idx(L, j, k), hi, lo);
+            bf.xL[fo] = r_; bf.xL[nx + fo] = mu_; bf.xL[2 * nx + fo] = mv; bf.xL[3 * nx + fo] = mw;
+            bf.xL[4 * nx + fo] = P_ / kc::K_1 + T(0.5) * (mu_ * mu_ + mv * mv + mw * mw) / r_;
+        } else if (!upper) { // periodic x, the reference's z rule (:94-109)
+            ghost_value(u, fs, FSL_CELL(g.idx(1, j, k), fs), false, false, gv);
+            edge_state<T, 0, true>(g, u, g.idx(L, j, k), gv, o);
 #pragma unroll
-            for (int q = 0; q < 5; q++) bf.x0[q * nx + FSL_FACE(fo, nx)] = hi[q];
-            recon_at<T, 0>(g, u, g.idx(1, j, k), hi, lo);
+            for (int q = 0; q < 5; q++) bf.x0[q * nx + fo] = o[q];
+        } else {
+            ghost_value(u, fs, FSL_CELL(g.idx(L, j, k), fs), false, false, gv);
+            edge_state<T, 0, false>(g, u, g.idx(1, j, k), gv, o);
 #pragma unroll
-            for (int q = 0; q < 5; q++) bf.xL[q * nx + FSL_FACE(fo, nx)] = lo[q];
+            for (int q = 0; q < 5; q++) bf.xL[q * nx + fo] = o[q];
         }
     } else if ((t -= nx) < ny) { // :75-90
-        const int i = (int)(t / D) + 1, k = (int)(t % D) + 1;
-        recon_at<T, 1>(g, u, g.idx(i, 1, k), hi, lo);
+        const unsigned r = (unsigned)t, q_ = r / (unsigned)D;
+        const int i = (int)q_ + 1, k = (int)(r - q_ * (unsigned)D) + 1;
+        const long long c = g.idx(i, upper ? H : 1, k), fo = FSL_FACE(t, ny);
+        ghost_value(u, fs, FSL_CELL(c, fs), spatial, false, gv);
+        if (upper) edge_state<T, 1, true>(g, u, c, gv, o);
+        else edge_state<T, 1, false>(g, u, c, gv, o);
+        T *dst = upper ? bf.yH : bf.y0;
 #pragma unroll
-        for (int q = 0; q < 5; q++) bf.y0[q * ny + FSL_FACE(t, ny)] = (q == 2 && spatial) ? -lo[q] : lo[q];
-        recon_at<T, 1>(g, u, g.idx(i, H, k), hi, lo);
-#pragma unroll
-        for (int q = 0; q < 5; q++) bf.yH[q * ny + FSL_FACE(t, ny)] = (q == 2 && spatial) ? -hi[q] : hi[q];
+        for (int q = 0; q < 5; q++) dst[q * ny + fo] = (q == 2 && spatial) ? -o[q] : o[q];
     } else if ((t -= ny) < nz) { // :94-109
-        const int i = (int)(t / H) + 1, j = (int)(t % H) + 1;
-        recon_at<T, 2>(g, u, g.idx(i, j, D), hi, lo);
+        const unsigned r = (unsigned)t, q_ = r / (unsigned)H;
+        const int i = (int)q_ + 1, j = (int)(r - q_ * (unsigned)H) + 1;
+        const long long fo = FSL_FACE(t, nz);
+        if (!upper) {
+            ghost_value(u, fs, FSL_CELL(g.idx(i, j, 1), fs), false, false, gv);
+            edge_state<T, 2, true>(g, u, g.idx(i, j, D), gv, o);
+        } else {
+            ghost_value(u, fs, FSL_CELL(g.idx(i, j, D), fs), false, false, gv);
+            edge_state<T, 2, false>(g, u, g.idx(i, j, 1), gv, o);
+        }
+        T *dst = upper ? bf.zD : bf.z0;
 #pragma unroll
-        for (int q = 0; q < 5; q++) bf.z0[q * nz + FSL_FACE(t, nz)] = hi[q];
-        recon_at<T, 2>(g, u, g.idx(i, j, 1), hi, lo);
-#pragma unroll
-        for (int q = 0; q < 5; q++) bf.zD[q * nz + FSL_FACE(t, nz)] = lo[q];
+        for (int q = 0; q < 5; q++) dst[q * nz + fo] = o[q];
     }
 }
 
+// The boundary pass before a fused stage: the ghost layer of u and the outer
+// states of the boundary faces, in one launch -- the faces form the ghost values
+// they need from the interior, so neither waits for the other (two dependent
+// launches of 5 and 9 us at 100x80x35 before).
 template <typename T>
-__global__ void k_bface(Grid g, int setup, int BL_HIG, Disturb d, const double *__restrict__ u, BF<T> bf)
+__global__ void __launch_bounds__(128) k_boundary(Grid g, int setup, int BL_HIG, Disturb d, double *__restrict__ u,
+                                                  BF<T> bf)
 {
-    const long long n = (long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) bface_one<T>(g, setup, BL_HIG, d, u, bf, t);
+    const long long nf = (long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H;
+    const bool spatial = setup == FSL_SETUP_SPATIAL;
+    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 2 * nf) {
+        const bool upper = t >= nf;
+        bface_one<T>(g, spatial, BL_HIG, d, u, bf, upper ? t - nf : t, upper);
+    } else if ((t -= 2 * nf) < ghost_cells(g)) {
+        ghost_cell(g, spatial, u, t);
+    }
 }
 
 template <typename T, int TJE, bool PPM = false> struct Smem {
@@ -700,12 +821,13 @@ int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, doubl
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <typename T> void launch_bface_t(Ctx &c, const double *cur, const Disturb &d, BF<T> bf)
+template <typename T> void launch_boundary_t(Ctx &c, double *cur, const Disturb &d, BF<T> bf)
 {
     const Grid &g = c.g;
-    const long long n = (long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H;
+    const long long n =
+        2 * ((long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H) + ghost_cells(g);
     prof_begin(c, FSL_K_BC);
-    k_bface<T><<<(unsigned)((n + 127) / 128), 128, 0, c.stream>>>(g, c.k.setup, c.k.BL_HIG, d, cur, bf);
+    k_boundary<T><<<(unsigned)((n + 127) / 128), 128, 0, c.stream>>>(g, c.k.setup, c.k.BL_HIG, d, cur, bf);
     prof_end(c, FSL_K_BC, 1);
 }
 
