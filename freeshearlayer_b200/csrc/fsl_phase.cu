@@ -42,20 +42,40 @@ __global__ void k_ghost(Grid g, int setup, double *__restrict__ u)
     if (t < stage::ghost_cells(g)) stage::ghost_cell(g, setup == FSL_SETUP_SPATIAL, u, t);
 }
 
+// Blocks of the per-phase kernels: kPlaneThreads consecutive entries of one
+// plane's nb x nc list, so short and ragged rows fill their warps (rows of 40
+// left 24 of every 64 lanes idle); block -> (plane a, row b, column c).
+// ---------------------------------------------------------------------------
+constexpr int kPlaneThreads = 128;
+__host__ __device__ inline unsigned plane_blocks(int nb, int nc)
+{
+    return ((unsigned)nb * (unsigned)nc + kPlaneThreads - 1) / kPlaneThreads;
+}
+__device__ __forceinline__ bool plane_cell(int nb, int nc, unsigned block, int &a, int &b, int &c)
+{
+    const unsigned per = plane_blocks(nb, nc), p = block / per;
+    const unsigned t = (block - p * per) * kPlaneThreads + threadIdx.x, r = t / (unsigned)nc;
+    a = (int)p;
+    b = (int)r;
+    c = (int)(t - r * (unsigned)nc);
+    return b < nb;
+}
+
 // ---------------------------------------------------------------------------
 // A2 reconstruction (src/reconstruction.c:26-345): one thread per interior
 // cell, all three sweeps, six face states written to the face arrays.  With
 // PPM, a sweep whose four neighbours exist (the cell is not next to the
-// domain boundary in that direction) uses ppm_* instead.
+// domain boundary in that direction) uses ppm_* instead.  FP64 arithmetic in a
+// chain of three sweeps: five blocks an SM (102 registers) where 132 registers
+// left three, and full warps; 96x72x40 29 -> 20 us with both.
 // ---------------------------------------------------------------------------
 template <bool PPM>
-__global__ void __launch_bounds__(128) k_recon(Grid g, const double *__restrict__ u, Faces f)
+__global__ void __launch_bounds__(kPlaneThreads, 5) k_recon(Grid g, const double *__restrict__ u, Faces f)
 {
     const int L = g.L, H = g.H, D = g.D;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int i = blockIdx.z + 1;
-    if (k > D || j > H) return;
+    int i, j, k;
+    if (!plane_cell(H, D, blockIdx.x, i, j, k)) return;
+    i++; j++; k++;
     const long long fs = g.fstride;
     const long long c0 = g.idx(i, j, k);
     if (!FSL_SPAN(c0, -g.pi, g.pi, fs)) return; // the one-neighbour stencil in x, the widest
@@ -130,7 +150,7 @@ __global__ void k_ifbc(Grid g, int setup, int BL_HIG, Disturb d, Faces f)
     const bool spatial = (setup == FSL_SETUP_SPATIAL);
     typedef Kc<double> kc;
     if (t < nx) {
-        const int j = (int)(t / D), k = (int)(t % D);
+        const int j = (int)((unsigned)t / (unsigned)D), k = (int)((unsigned)t % (unsigned)D);
         const long long f0 = ixf(L, H, D, 0, j, k), fL = ixf(L, H, D, L, j, k);
         if (spatial) {
             const double P = 100000., R = 1.0;
@@ -166,7 +186,7 @@ __global__ void k_ifbc(Grid g, int setup, int BL_HIG, Disturb d, Faces f)
             }
         }
     } else if ((t -= nx) < ny) { // :75-90
-        const int i = (int)(t / D), k = (int)(t % D);
+        const int i = (int)((unsigned)t / (unsigned)D), k = (int)((unsigned)t % (unsigned)D);
         const long long f0 = iyf(L, H, D, i, 0, k), fH = iyf(L, H, D, i, H, k);
 #pragma unroll
         for (int q = 0; q < 5; q++) {
@@ -179,7 +199,7 @@ __global__ void k_ifbc(Grid g, int setup, int BL_HIG, Disturb d, Faces f)
             }
         }
     } else if ((t -= ny) < nz) { // :94-109
-        const int i = (int)(t / H), j = (int)(t % H);
+        const int i = (int)((unsigned)t / (unsigned)H), j = (int)((unsigned)t % (unsigned)H);
         const long long f0 = izf(L, H, D, i, j, 0), fD = izf(L, H, D, i, j, D);
 #pragma unroll
         for (int q = 0; q < 5; q++) {
@@ -190,22 +210,26 @@ __global__ void k_ifbc(Grid g, int setup, int BL_HIG, Disturb d, Faces f)
 }
 
 // ---------------------------------------------------------------------------
-// A4 fluxes (src/fluxes.c:57-571): one thread per face of direction N.
-// The flux overwrites the minus-side state array, as in the reference.
+// A4 fluxes (src/fluxes.c:57-571): one thread per face, the three directions in
+// one launch.  The flux overwrites the minus-side state array, as in the
+// reference.  Bound by FP64 arithmetic and the latency of its chain: the eight
+// tangential reciprocals are formed without a branch (rcp_rn, divisions when one
+// is out of its range).  96x72x40: 92 us in three launches -> 44 us (four blocks
+// an SM 50 us, six 45).
 // ---------------------------------------------------------------------------
+__device__ __noinline__ double inverse(double x) { return 1. / x; }
+
 // sgs: FSL_SGS_STATIC forms the face viscosity from the face gradients and
 // the two cells' densities (src/fluxes.c:193-205, :362-374, :533-545),
 // FSL_SGS_NONE uses zero, any other mode the mu_SGS field.
 template <int N>
-__global__ void __launch_bounds__(128) k_flux(Grid g, Consts kc, const double *__restrict__ u,
-                                              const double *__restrict__ mu, Faces f, int sgs)
+__device__ __forceinline__ void flux_face(const Grid &g, const Consts &kc, const double *__restrict__ u,
+                                          const double *__restrict__ mu, const Faces &f, int sgs, unsigned block)
 {
-    const int L = g.L, H = g.H, D = g.D;
-    const int na = L + (N == 1), nb = H + (N == 2), nc = D + (N == 3);
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y * blockDim.y + threadIdx.y;
-    const int a = blockIdx.z;
-    if (c >= nc || b >= nb || a >= na) return;
+    const int H = g.H, D = g.D;
+    const int nb = H + (N == 2), nc = D + (N == 3);
+    int a, b, c;
+    if (!plane_cell(nb, nc, block, a, b, c)) return;
     const long long fs = g.fstride;
     long long fi;
     double *const *mS;
@@ -231,7 +255,7 @@ __global__ void __launch_bounds__(128) k_flux(Grid g, Consts kc, const double *_
     const long long minus = plus - dn;
     // the neighbours read: plus and minus, each with both tangential offsets
     if (!FSL_SPAN(plus, -dn - (dt1 > dt2 ? dt1 : dt2), dt1 > dt2 ? dt1 : dt2, fs)) return;
-    fi = FSL_FACE(fi, (long long)na * nb * nc);
+    fi = FSL_FACE(fi, (long long)(g.L + (N == 1)) * nb * nc);
     double Lm[5], Rp[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) { Lm[q] = mS[q][fi]; Rp[q] = pS[q][fi]; }
@@ -240,12 +264,29 @@ __global__ void __launch_bounds__(128) k_flux(Grid g, Consts kc, const double *_
     double vp[3], vm[3], Tp, Tm;
     vel_div(u[plus], u[fs + plus], u[2 * fs + plus], u[3 * fs + plus], u[4 * fs + plus], vp, Tp);
     vel_div(u[minus], u[fs + minus], u[2 * fs + minus], u[3 * fs + minus], u[4 * fs + minus], vm, Tm);
-    // tangential neighbours: P/M = plus/minus cell, h/l = +/- tangential offset
-    double Ph1[3], Mh1[3], Pl1[3], Ml1[3], Ph2[3], Mh2[3], Pl2[3], Ml2[3];
-#define LOADV(dst, at) vel_rcp(u[at], u[fs + (at)], u[2 * fs + (at)], u[3 * fs + (at)], dst)
-    LOADV(Ph1, plus + dt1); LOADV(Mh1, minus + dt1); LOADV(Pl1, plus - dt1); LOADV(Ml1, minus - dt1);
-    LOADV(Ph2, plus + dt2); LOADV(Mh2, minus + dt2); LOADV(Pl2, plus - dt2); LOADV(Ml2, minus - dt2);
-#undef LOADV
+    // tangential neighbours: the plus and the minus cell's, at +/- both offsets,
+    // with the rounded reciprocal density of src/fluxes.c:124-142
+    const long long at[8] = {plus + dt1, minus + dt1, plus - dt1, minus - dt1,
+                             plus + dt2, minus + dt2, plus - dt2, minus - dt2};
+    double ru[8];
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const double r = u[at[q]];
+        ru[q] = rcp_rn(r);
+        ok = ok && range_ok(r) && !ones(r);
+    }
+    if (!ok) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) ru[q] = inverse(u[at[q]]);
+    }
+    double s1[3], s2[3]; // sums over the two faces' cells of the tangential differences
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const double *m = u + (q + 1) * fs;
+        s1[q] = m[at[0]] * ru[0] + m[at[1]] * ru[1] - m[at[2]] * ru[2] - m[at[3]] * ru[3];
+        s2[q] = m[at[4]] * ru[4] + m[at[5]] * ru[5] - m[at[6]] * ru[6] - m[at[7]] * ru[7];
+    }
     // g[a][b] = d u_a / d x_b
     double gr[3][3];
     const int n0 = N - 1;
@@ -254,8 +295,8 @@ __global__ void __launch_bounds__(128) k_flux(Grid g, Consts kc, const double *_
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         gr[q][n0] = (vp[q] - vm[q]) * rdn;
-        gr[q][t1] = (Ph1[q] + Mh1[q] - Pl1[q] - Ml1[q]) * rt1;
-        gr[q][t2] = (Ph2[q] + Mh2[q] - Pl2[q] - Ml2[q]) * rt2;
+        gr[q][t1] = s1[q] * rt1;
+        gr[q][t2] = s2[q] * rt2;
     }
     // SGS viscosity at the face: x uses the two adjacent cells (:191); the y
     // and z sweeps average the plus cell with its x-neighbour (:360, :531).
@@ -269,19 +310,28 @@ __global__ void __launch_bounds__(128) k_flux(Grid g, Consts kc, const double *_
     for (int q = 0; q < 5; q++) mS[q][fi] = F[q];
 }
 
+// blocks [0, bx) the x faces, [bx, by) the y faces, the others the z faces
+__global__ void __launch_bounds__(kPlaneThreads, 5) k_flux(Grid g, Consts kc, const double *__restrict__ u,
+                                                        const double *__restrict__ mu, Faces f, int sgs, unsigned bx,
+                                                        unsigned by)
+{
+    if (blockIdx.x < bx) flux_face<1>(g, kc, u, mu, f, sgs, blockIdx.x);
+    else if (blockIdx.x < by) flux_face<2>(g, kc, u, mu, f, sgs, blockIdx.x - bx);
+    else flux_face<3>(g, kc, u, mu, f, sgs, blockIdx.x - by);
+}
+
 // ---------------------------------------------------------------------------
 // A7 TVD Runge-Kutta (src/evolution.c:15-245).  mode: 1..3 = RK3 stage,
 // 4 = the nStages == 2 chain of stage 1, 5 = the chain of stage 2 (RK2 stage
 // 2 followed by RK3 stage 2 on the updated U, src/evolution.c:19-23).
 // ---------------------------------------------------------------------------
-__global__ void k_evolution(Grid g, int mode, const DevScalars *__restrict__ ds, double *__restrict__ U,
+__global__ void __launch_bounds__(kPlaneThreads) k_evolution(Grid g, int mode, const DevScalars *__restrict__ ds, double *__restrict__ U,
                             double *__restrict__ Up, Faces f)
 {
     const int L = g.L, H = g.H, D = g.D;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int i = blockIdx.z + 1;
-    if (k > D || j > H) return;
+    int i, j, k;
+    if (!plane_cell(H, D, blockIdx.x, i, j, k)) return;
+    i++; j++; k++;
     const double dtx = ds->dtx, dty = ds->dty, dtz = ds->dtz;
     const double one_third = 1. / 3., two_thirds = 2. / 3.;
     const long long fs = g.fstride, c = FSL_CELL(g.idx(i, j, k), fs);
@@ -574,11 +624,6 @@ __global__ void k_plane_sums_final(int n, int nseg, const double *__restrict__ p
     rows[t] = x;
 }
 
-inline dim3 cells_grid(const Grid &g, dim3 b, int ni, int nj, int nk)
-{
-    return dim3((nk + b.x - 1) / b.x, (nj + b.y - 1) / b.y, ni);
-}
-
 } // namespace
 
 // ---- launchers -------------------------------------------------------------
@@ -595,10 +640,10 @@ void launch_ghost(Ctx &c, double *cur)
 void launch_recon(Ctx &c, const double *cur)
 {
     const Grid &g = c.g;
-    dim3 b(32, 4, 1);
+    const unsigned n = (unsigned)g.L * plane_blocks(g.H, g.D);
     prof_begin(c, FSL_K_RECON);
-    if (c.p.recon == FSL_RECON_PPM) k_recon<true><<<cells_grid(g, b, g.L, g.H, g.D), b, 0, c.stream>>>(g, cur, c.f);
-    else k_recon<false><<<cells_grid(g, b, g.L, g.H, g.D), b, 0, c.stream>>>(g, cur, c.f);
+    if (c.p.recon == FSL_RECON_PPM) k_recon<true><<<n, kPlaneThreads, 0, c.stream>>>(g, cur, c.f);
+    else k_recon<false><<<n, kPlaneThreads, 0, c.stream>>>(g, cur, c.f);
     prof_end(c, FSL_K_RECON, 1);
 }
 
@@ -614,12 +659,12 @@ void launch_ifbc(Ctx &c, const Disturb &d)
 void launch_fluxes(Ctx &c, const double *cur)
 {
     const Grid &g = c.g;
-    dim3 b(32, 4, 1);
+    const unsigned bx = (unsigned)(g.L + 1) * plane_blocks(g.H, g.D);
+    const unsigned by = bx + (unsigned)g.L * plane_blocks(g.H + 1, g.D);
+    const unsigned n = by + (unsigned)g.L * plane_blocks(g.H, g.D + 1);
     prof_begin(c, FSL_K_FLUX);
-    k_flux<1><<<cells_grid(g, b, g.L + 1, g.H, g.D), b, 0, c.stream>>>(g, c.k, cur, c.mu, c.f, c.p.sgs);
-    k_flux<2><<<cells_grid(g, b, g.L, g.H + 1, g.D), b, 0, c.stream>>>(g, c.k, cur, c.mu, c.f, c.p.sgs);
-    k_flux<3><<<cells_grid(g, b, g.L, g.H, g.D + 1), b, 0, c.stream>>>(g, c.k, cur, c.mu, c.f, c.p.sgs);
-    prof_end(c, FSL_K_FLUX, 3);
+    k_flux<<<n, kPlaneThreads, 0, c.stream>>>(g, c.k, cur, c.mu, c.f, c.p.sgs, bx, by);
+    prof_end(c, FSL_K_FLUX, 1);
 }
 
 void launch_evolution(Ctx &c, int nstages, int stage)
@@ -627,9 +672,9 @@ void launch_evolution(Ctx &c, int nstages, int stage)
     const Grid &g = c.g;
     int mode = stage >= 3 ? 3 : stage;
     if (nstages == 2) mode = (stage == 1) ? 4 : 5;
-    dim3 b(32, 4, 1);
+    const unsigned n = (unsigned)g.L * plane_blocks(g.H, g.D);
     prof_begin(c, FSL_K_EVOL);
-    k_evolution<<<cells_grid(g, b, g.L, g.H, g.D), b, 0, c.stream>>>(g, mode, c.ds, c.U, c.Up, c.f);
+    k_evolution<<<n, kPlaneThreads, 0, c.stream>>>(g, mode, c.ds, c.U, c.Up, c.f);
     prof_end(c, FSL_K_EVOL, 1);
 }
 
