@@ -314,6 +314,7 @@ template <typename T> struct Args {
     unsigned int *status;   // bit 1 set on a non-positive output density (with co)
     int stage;
     int seg;
+    int split;
     // non-null (full-lane tile, temporal setup): also write the FP32 velocities
     // of `out`, ghost cells included, as the closure's velocity pass forms them
     float *vel;
@@ -445,9 +446,26 @@ __device__ __forceinline__ void ring_consts(const Smem<T, TJE, PPM> &s, const T 
     }
 }
 
+// The FP32 kernels' results depend in their last bits on where a march begins (its
+// prologue and its loop are compiled apart).  A march is therefore cut into `split`
+// parts for the SMs a small grid leaves idle without moving its beginning: a part
+// that begins inside computes WARM planes before the first it writes, so that all
+// it takes over -- the flux of face i - 1/2, the x sweep's state and the velocities
+// of plane i-1 -- was formed by the loop, and the cut shows in no bit.
+constexpr int WARM = 3;
+
+// First plane of part p of a march of n planes in `split` parts of equal cost, each
+// but the first paying for its WARM planes.
+__host__ __device__ inline long long part_begin(long long n, int p, int split)
+{
+    if (p == 0) return 0;
+    return n < WARM ? n : (n + WARM * (split - 1)) * p / split - (long long)WARM * (p - 1);
+}
+
 // SST: static Smagorinsky (the face viscosity from the face gradients and the
-// two cells' densities; no mu field is read).
-template <typename T, int TJE, int MINB, bool PPM, bool SST>
+// two cells' densities; no mu field is read).  SPLIT: block z is part z % a.split
+// of segment z / a.split.
+template <typename T, int TJE, int MINB, bool PPM, bool SST, bool SPLIT = false>
 __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Args<T> a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -459,8 +477,15 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     const int r = threadIdx.y, l = threadIdx.x;
     const int j = blockIdx.y * TJ + r;
     const int k = blockIdx.x * 30 + l;
-    const int i0 = 1 + blockIdx.z * a.seg;
-    const int i1 = min(L, i0 + a.seg - 1);
+    int i0 = 1 + (SPLIT ? blockIdx.z / a.split : blockIdx.z) * a.seg;
+    int i1 = min(L, i0 + a.seg - 1), iw = i0; // iw: the first plane written
+    if constexpr (SPLIT) {
+        const int n = i1 - i0 + 1, p = (int)(blockIdx.z % a.split), b = i0;
+        iw = b + (int)part_begin(n, p, a.split);
+        i1 = b + (int)part_begin(n, p + 1, a.split) - 1;
+        if (iw > i1) return;
+        i0 = max(b, iw - WARM);
+    }
     const bool live = (j <= H + 1) && (k <= D + 1);
     const bool inter = live && r >= 1 && r <= TJE - 2 && l >= 1 && l <= 30 && j <= H && k <= D;
     const bool ycol = live && l >= 1 && l <= 30 && k <= D;     // column takes part in y faces
@@ -575,7 +600,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
             if (sizeof(T) != 8) {
 #pragma unroll
                 for (int q = 0; q < 5; q++) base[q] = cu[q * fs + c];
-                if (a.stage != 1) {
+                if (a.stage != 1 && (!SPLIT || i >= iw)) { // (the planes before iw are another block's)
 #pragma unroll
                     for (int q = 0; q < 5; q++) unv[q] = a.un[q * fs + c];
                 }
@@ -719,7 +744,7 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
         }
         __syncthreads();
         // (f) divergence and stage combination (src/evolution.c:29-161), FP64
-        if (inter) {
+        if (inter && (!SPLIT || i >= iw)) {
             const long long c = FSL_CELL(cj + (long long)i * g.pi, fs);
             const T *Uc = s.U[q0][r + HW][l + HW];
             (void)Uc;
@@ -797,6 +822,15 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     }
 }
 
+// Parts of each march: as many as fill the SMs the grid's blocks leave idle, down
+// to two planes a part.  Used where no bit may change (the FP32 PPM tile).  Three
+// stages at 64x32x32 983 -> 172 us, 128x64x64 993 -> 395 us, 110x48x80 998 -> 333 us;
+// with more than half the SMs at work a second part has no SM to run on.
+inline int march_split(const Grid &g, int nb, int seg, int sms)
+{
+    return std::max(1, std::min(sms / nb, std::min(seg, g.L) / 2));
+}
+
 template <typename T, int TJE, int MINB, bool PPM = false, bool SST = false>
 int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, double *out, const T *mu, BF<T> bf,
                    bool courant, int seg = 0)
@@ -810,11 +844,24 @@ int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, doubl
     a.status = &c.ds->status;
     a.seg = seg > 0 ? seg : c.stage_seg;
     a.vel = nullptr;
+    a.split = 1;
     const size_t smem = sizeof(Smem<T, TJE, PPM>);
     static std::atomic<uint64_t> attr{0};
     if (!smem_limit_once((const void *)k_stage<T, TJE, MINB, PPM, SST>, smem, attr)) return -1;
     dim3 b(32, TJE, 1);
     dim3 gr((g.D + 29) / 30, (g.H + TJE - 3) / (TJE - 2), (g.L + a.seg - 1) / a.seg);
+    if constexpr (sizeof(T) == 4 && PPM && TJE == 16) {
+        const long long nb = (long long)gr.x * gr.y * gr.z;
+        if (nb * 2 <= c.sms && (a.split = march_split(g, (int)nb, a.seg, c.sms)) > 1) {
+            static std::atomic<uint64_t> attr_split{0};
+            if (!smem_limit_once((const void *)k_stage<T, TJE, MINB, PPM, SST, true>, smem, attr_split)) return -1;
+            gr.z *= a.split;
+            prof_begin(c, FSL_K_STAGE);
+            k_stage<T, TJE, MINB, PPM, SST, true><<<gr, b, smem, c.stream>>>(g, c.k, a);
+            prof_end(c, FSL_K_STAGE, 1);
+            return cudaGetLastError() == cudaSuccess ? 0 : -1;
+        }
+    }
     prof_begin(c, FSL_K_STAGE);
     k_stage<T, TJE, MINB, PPM, SST><<<gr, b, smem, c.stream>>>(g, c.k, a);
     prof_end(c, FSL_K_STAGE, 1);

@@ -42,7 +42,9 @@ namespace wide {
 using stage::Args;
 using stage::BF;
 using stage::load5;
+using stage::part_begin;
 using stage::recon_at;
+using stage::WARM;
 
 constexpr int WJ = 16;  // tile rows (warps)
 constexpr int WK = 32;  // tile columns (lanes)
@@ -241,10 +243,11 @@ __device__ __forceinline__ void halo_sweeps(Smem<T> &s, const Args<T> &a, int p,
 }
 
 // Block b of a domain's stage launch of nb blocks: its share of the
-// (tile, plane) pairs, and with a.co the Courant maximum of what it wrote.
-template <typename T, bool SST>
+// (tile, plane) pairs (SPLIT: part `part` of `split` parts of it), and with a.co
+// the Courant maximum of what it wrote.
+template <typename T, bool SST, bool SPLIT>
 __device__ __forceinline__ void wide_block(Smem<T> &s, const Grid &g, const Consts &kc, const Args<T> &a, int b,
-                                           int nb)
+                                           int nb, int part, int split)
 {
     const int L = g.L, H = g.H, D = g.D;
     const int t = threadIdx.x, r = t >> 5, l = t & 31;
@@ -288,6 +291,11 @@ __device__ __forceinline__ void wide_block(Smem<T> &s, const Grid &g, const Cons
         end = total * (b + 1) / nb;
     }
     const long long Lt = L - Hd, nhead = ntiles * Hd;
+    long long from = pos, to = end; // the units this block writes
+    if constexpr (SPLIT) {
+        from = pos + part_begin(end - pos, part, split);
+        to = pos + part_begin(end - pos, part + 1, split);
+    }
     while (pos < end) {
         long long tile, run;
         int i0;
@@ -301,8 +309,18 @@ __device__ __forceinline__ void wide_block(Smem<T> &s, const Grid &g, const Cons
             i0 = (int)(Hd + v % Lt) + 1;
             run = Lt - (v % Lt);
         }
-        const int i1 = i0 + (int)min(run, end - pos) - 1;
-        pos += i1 - i0 + 1;
+        int i1 = i0 + (int)min(run, end - pos) - 1;
+        int iw = i0; // the first plane written
+        if constexpr (SPLIT) {
+            const long long lo = max(from - pos, 0LL), hi = min(to - pos, (long long)(i1 - i0 + 1));
+            pos += i1 - i0 + 1;
+            if (lo >= hi) continue;
+            iw = i0 + (int)lo;
+            i1 = i0 + (int)hi - 1;
+            i0 = max(i0, iw - WARM);
+        } else {
+            pos += i1 - i0 + 1;
+        }
         const int k0 = (int)(tile % ntk) * WK + 1, j0 = (int)(tile / ntk) * WJ + 1;
         const int j = j0 + r, k = k0 + l;
         // temporal setup (periodic z): the ring's columns beyond the ghost
@@ -411,7 +429,7 @@ __device__ __forceinline__ void wide_block(Smem<T> &s, const Grid &g, const Cons
                 const long long c = FSL_CELL(cj + (long long)i * g.pi, fs);
 #pragma unroll
                 for (int q = 0; q < 5; q++) base[q] = cu[q * fs + c];
-                if (a.stage != 1) {
+                if (a.stage != 1 && (!SPLIT || i >= iw)) { // (the planes before iw are another block's)
 #pragma unroll
                     for (int q = 0; q < 5; q++) unv[q] = a.un[q * fs + c];
                 }
@@ -541,7 +559,7 @@ __device__ __forceinline__ void wide_block(Smem<T> &s, const Grid &g, const Cons
             __syncthreads();
             // (d) divergence and stage combination (src/evolution.c:29-161):
             // the divergence in FP32, the combination in FP64
-            if (own) {
+            if (own && (!SPLIT || i >= iw)) {
                 if (l == 0) {
 #pragma unroll
                     for (int q = 0; q < 5; q++) Fzm[q] = s.FzL[r][q];
@@ -741,6 +759,7 @@ struct WideWork {
     const int *start;
     int s_begin, s_end;
     int courant; // stage 3 accumulates the Courant maximum
+    int split;   // m0: parts of a block's share
     GridBarrier bar;
 };
 
@@ -759,6 +778,7 @@ __device__ __forceinline__ Args<float> member_args(const WideMember &M, int st, 
     a.status = M.status;
     a.stage = st;
     a.seg = 0;
+    a.split = 1;
     a.vel = st == 3 ? M.vel : nullptr;
     return a;
 }
@@ -766,15 +786,20 @@ __device__ __forceinline__ Args<float> member_args(const WideMember &M, int st, 
 // MULTI = false: one stage of the domain w.m0, block x its block x (its
 // descriptor stays in the parameter space).  MULTI = true: the work list.
 // Both instantiate the same block code (wide_block), so a domain stepped
-// alone and in a multi-domain launch computes the same values.
-template <bool SST, bool MULTI>
+// alone and in a multi-domain launch computes the same values.  SPLIT: block x is
+// part x % split of block x / split.
+template <bool SST, bool MULTI, bool SPLIT = false>
 __global__ void __launch_bounds__(NT, 1) k_wide(WideWork w)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     Smem<float> &s = *reinterpret_cast<Smem<float> *>(smraw);
-    if constexpr (!MULTI) {
-        wide_block<float, SST>(s, w.m0.g, w.m0.kc, member_args(w.m0, w.s_begin, w.courant != 0), blockIdx.x,
-                               w.m0.nb);
+    if constexpr (SPLIT) {
+        const int b = (int)blockIdx.x / w.split;
+        wide_block<float, SST, true>(s, w.m0.g, w.m0.kc, member_args(w.m0, w.s_begin, w.courant != 0), b, w.m0.nb,
+                                     (int)blockIdx.x - b * w.split, w.split);
+    } else if constexpr (!MULTI) {
+        wide_block<float, SST, false>(s, w.m0.g, w.m0.kc, member_args(w.m0, w.s_begin, w.courant != 0), blockIdx.x,
+                                      w.m0.nb, 0, 1);
     } else {
         for (int st = w.s_begin; st <= w.s_end; st++) {
             const int i0 = w.start[blockIdx.x], i1 = w.start[blockIdx.x + 1];
@@ -792,7 +817,7 @@ __global__ void __launch_bounds__(NT, 1) k_wide(WideWork w)
                     sa = member_args(sm, st, w.courant != 0);
                 }
                 __syncthreads();
-                wide_block<float, SST>(s, sm.g, sm.kc, sa, b, sm.nb);
+                wide_block<float, SST, false>(s, sm.g, sm.kc, sa, b, sm.nb, 0, 1);
             }
             if (st == w.s_end) break;
             // the stage's outputs (ghost cells included) complete before the next reads them
@@ -837,10 +862,19 @@ inline WideMember wide_member(const Ctx &c, const float *mu, BF<float> bf, int s
     return m;
 }
 
-template <bool SST, bool MULTI> inline bool wide_attr()
+// Parts of each block's share when a domain is stepped alone: as many as fill
+// the SMs that wide_blocks leaves idle, down to two planes a part.  Three stages at
+// 64x32x32 287 -> 112 us, 128x64x64 291 -> 212 us, 110x48x80 329 -> 228 us.
+inline int wide_split(const Grid &g, int nb, int sms)
+{
+    const long long units = (long long)((g.D + WK - 1) / WK) * ((g.H + WJ - 1) / WJ) * g.L;
+    return (int)std::max(1LL, std::min((long long)(sms / nb), units / nb / 2));
+}
+
+template <bool SST, bool MULTI, bool SPLIT = false> inline bool wide_attr()
 {
     static std::atomic<uint64_t> attr{0};
-    return smem_limit_once((const void *)k_wide<SST, MULTI>, sizeof(Smem<float>), attr);
+    return smem_limit_once((const void *)k_wide<SST, MULTI, SPLIT>, sizeof(Smem<float>), attr);
 }
 
 // One stage of one domain (the FP32 bulk's fused stage with the reference
@@ -850,7 +884,7 @@ int launch_wide(Ctx &c, int stage, const double *cur, const double *un, double *
                 BF<float> bf, bool courant, float *vel)
 {
     (void)cur; (void)un; (void)out; // always U -> Up -> Uq -> U with U^n = U
-    if (!wide_attr<SST, false>()) return -1;
+    if (!wide_attr<SST, false>() || !wide_attr<SST, false, true>()) return -1;
     WideWork w{};
     w.m0 = wide_member(c, mu, bf, c.sms);
     w.m0.vel = vel;
@@ -860,8 +894,10 @@ int launch_wide(Ctx &c, int stage, const double *cur, const double *un, double *
     w.start = nullptr;
     w.s_begin = w.s_end = stage;
     w.courant = courant ? 1 : 0;
+    w.split = wide_split(c.g, w.m0.nb, c.sms);
     prof_begin(c, FSL_K_STAGE);
-    k_wide<SST, false><<<w.m0.nb, NT, sizeof(Smem<float>), c.stream>>>(w);
+    if (w.split > 1) k_wide<SST, false, true><<<w.m0.nb * w.split, NT, sizeof(Smem<float>), c.stream>>>(w);
+    else k_wide<SST, false><<<w.m0.nb, NT, sizeof(Smem<float>), c.stream>>>(w);
     prof_end(c, FSL_K_STAGE, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
