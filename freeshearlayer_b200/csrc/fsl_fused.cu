@@ -42,19 +42,19 @@ static Cut cut_tiles(const Grid &g, int sms, int tj, int tk, double start)
 static Cut ring_cut(const Grid &g, int sms, int tj) { return cut_tiles(g, sms, tj, 30, 1.2); }
 static Cut dir_cut(const Grid &g, int sms) { return cut_tiles(g, sms, dirs::WJ, dirs::WK, 2.0); }
 
-// The ring tile marches a plane of 14 x 30 cells in 11.2 us, the direction-split
-// kernel one of 4 x 32 in 5.1 us and 3 us a launch, whatever the grid (measured
+// The ring tile marches a plane of 14 x 30 cells in 10.8 us, the direction-split
+// kernel one of 4 x 32 in 4.95 us and 3 us a launch, whatever the grid (measured
 // from 24x16x16 to 256x128x128): per cell the ring is faster by half, but the
 // smaller tiles leave fewer SMs idle on small grids and no columns empty where
 // DEP is a multiple of 32, and on the temporal setup the direction split needs no
-// boundary passes (18 us a stage).  Per step, ring with its passes against
-// direction split: 64x32x32 197 / 102 us, 512x64x32 1448 / 933, 100x80x35
-// (spatial) 406 / 583, 256x128x128 3431 / 4064.
+// boundary pass (6 us a stage and more on large grids).  Per step, ring with its
+// passes against direction split: 64x32x32 163 / 107 us, 96x48x48 261 / 284,
+// 512x64x32 1288 / 924, 100x80x35 (spatial) 361 / 515, 256x128x128 3076 / 3553.
 bool stage_splits_directions(const Ctx &c)
 {
     if (c.p.recon != FSL_RECON_CHARMINMOD || c.stage_tje != 0 || c.seg_set) return false;
-    const double passes = c.p.setup == FSL_SETUP_TEMPORAL ? 18. : 0.;
-    return 3. + 5.1 * dir_cut(c.g, c.sms).cost < 11.2 * ring_cut(c.g, c.sms, 14).cost + passes;
+    const double pass = c.p.setup == FSL_SETUP_TEMPORAL ? 6. : 0.;
+    return 3. + 4.95 * dir_cut(c.g, c.sms).cost < 10.8 * ring_cut(c.g, c.sms, 14).cost + pass;
 }
 
 template <bool SST>
