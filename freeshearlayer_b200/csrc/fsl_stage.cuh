@@ -314,7 +314,6 @@ template <typename T> struct Args {
     unsigned int *status;   // bit 1 set on a non-positive output density (with co)
     int stage;
     int seg;
-    int split;
     // non-null (full-lane tile, temporal setup): also write the FP32 velocities
     // of `out`, ghost cells included, as the closure's velocity pass forms them
     float *vel;
@@ -463,8 +462,9 @@ __host__ __device__ inline long long part_begin(long long n, int p, int split)
 }
 
 // SST: static Smagorinsky (the face viscosity from the face gradients and the
-// two cells' densities; no mu field is read).  SPLIT: block z is part z % a.split
-// of segment z / a.split.
+// two cells' densities; no mu field is read).  SPLIT: the blocks of a segment along
+// z are its parts (their number follows from the grid: one more argument made the
+// FP64 kernels' compilation spill, 1.6 % and with PPM 4 % of their time).
 template <typename T, int TJE, int MINB, bool PPM, bool SST, bool SPLIT = false>
 __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Args<T> a)
 {
@@ -477,12 +477,13 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
     const int r = threadIdx.y, l = threadIdx.x;
     const int j = blockIdx.y * TJ + r;
     const int k = blockIdx.x * 30 + l;
-    int i0 = 1 + (SPLIT ? blockIdx.z / a.split : blockIdx.z) * a.seg;
+    const int split = SPLIT ? (int)gridDim.z / ((L + a.seg - 1) / a.seg) : 1;
+    int i0 = 1 + (SPLIT ? blockIdx.z / split : blockIdx.z) * a.seg;
     int i1 = min(L, i0 + a.seg - 1), iw = i0; // iw: the first plane written
     if constexpr (SPLIT) {
-        const int n = i1 - i0 + 1, p = (int)(blockIdx.z % a.split), b = i0;
-        iw = b + (int)part_begin(n, p, a.split);
-        i1 = b + (int)part_begin(n, p + 1, a.split) - 1;
+        const int n = i1 - i0 + 1, p = (int)blockIdx.z % split, b = i0;
+        iw = b + (int)part_begin(n, p, split);
+        i1 = b + (int)part_begin(n, p + 1, split) - 1;
         if (iw > i1) return;
         i0 = max(b, iw - WARM);
     }
@@ -844,7 +845,6 @@ int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, doubl
     a.status = &c.ds->status;
     a.seg = seg > 0 ? seg : c.stage_seg;
     a.vel = nullptr;
-    a.split = 1;
     const size_t smem = sizeof(Smem<T, TJE, PPM>);
     static std::atomic<uint64_t> attr{0};
     if (!smem_limit_once((const void *)k_stage<T, TJE, MINB, PPM, SST>, smem, attr)) return -1;
@@ -852,10 +852,11 @@ int launch_stage_t(Ctx &c, int stage, const double *cur, const double *un, doubl
     dim3 gr((g.D + 29) / 30, (g.H + TJE - 3) / (TJE - 2), (g.L + a.seg - 1) / a.seg);
     if constexpr (sizeof(T) == 4 && PPM && TJE == 16) {
         const long long nb = (long long)gr.x * gr.y * gr.z;
-        if (nb * 2 <= c.sms && (a.split = march_split(g, (int)nb, a.seg, c.sms)) > 1) {
+        const int split = nb * 2 <= c.sms ? march_split(g, (int)nb, a.seg, c.sms) : 1;
+        if (split > 1) {
             static std::atomic<uint64_t> attr_split{0};
             if (!smem_limit_once((const void *)k_stage<T, TJE, MINB, PPM, SST, true>, smem, attr_split)) return -1;
-            gr.z *= a.split;
+            gr.z *= split;
             prof_begin(c, FSL_K_STAGE);
             k_stage<T, TJE, MINB, PPM, SST, true><<<gr, b, smem, c.stream>>>(g, c.k, a);
             prof_end(c, FSL_K_STAGE, 1);

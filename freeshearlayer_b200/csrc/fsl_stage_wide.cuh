@@ -778,7 +778,6 @@ __device__ __forceinline__ Args<float> member_args(const WideMember &M, int st, 
     a.status = M.status;
     a.stage = st;
     a.seg = 0;
-    a.split = 1;
     a.vel = st == 3 ? M.vel : nullptr;
     return a;
 }
