@@ -7,6 +7,7 @@
 
 #include "fsl_check.cuh"
 #include "fsl_internal.h"
+#include "fsl_phys.cuh"
 
 namespace fsl {
 namespace dyn {
@@ -223,9 +224,11 @@ __global__ void k_dyn_final(Grid g, Consts kc, const double *__restrict__ rho, c
 // per block whatever the grid.  This one reads the state once per block, keeps
 // everything else on chip (no scratch fields), and cuts the march so that the
 // blocks fill the SMs.  It is bound by the latency of shared memory, shuffles and
-// dependent arithmetic at 16 warps an SM (issue slots 42 % busy in FP64, 60 %
-// in FP32).  Measured: FP64 512x256x256 4.21 -> 3.15 ms, 64x32x32 177 -> 35 us;
-// FP32 203x97x75 195 -> 78 us.
+// dependent arithmetic at 16 warps an SM (issue slots 46 % busy in FP64, 60 %
+// in FP32).  The own row's summands come from registers, not shared memory, and
+// FP64 forms its two quotients without a branch (3.15 -> 3.00 ms).  Measured:
+// FP64 512x256x256 4.21 -> 3.00 ms, 64x32x32 177 -> 33 us; FP32 203x97x75 195 ->
+// 74 us.
 // ---------------------------------------------------------------------------
 constexpr int DYN_W = 16, DYN_J = DYN_W - 2, DYN_K = 28; // warps, output rows, output columns
 
@@ -234,11 +237,12 @@ template <typename T> struct DynSmem {
     T Q[DYN_W + 2][32][9];           // h times u v w uu uv uw vv vw ww of plane p
     T V[2][DYN_W + 2][32][3];        // velocities of planes p, p-1
     T F[2][DYN_W][32][3];            // filtered velocities of planes p-1, p-2
-    T A[DYN_W][32][6];               // h A of plane p-1
+    T A[DYN_W][6][32];               // h A of plane p-1
     // running x sums of the nine filters: FP64 in shared memory (own slots), as
     // registers they would spill at 128 a thread; FP32 in registers
     static constexpr bool XS = sizeof(T) == 8;
     T X[XS ? 18 : 1][DYN_W * 32];
+    T t0[XS ? 3 : 1][DYN_W * 32]; // the y pass of plane 0, kept as the sums are
 };
 
 template <typename T> __device__ __forceinline__ T sh_up(T v) { return __shfl_up_sync(0xffffffffu, v, 1); }
@@ -257,6 +261,26 @@ template <typename T> __device__ __forceinline__ T strain_of(const T (*d)[3], T 
     const T S21 = S[1], S31 = S[2], S32 = S[4];
     return sqrt(2 * (S[0] * S[0] + S[1] * S[1] + S[2] * S[2] + S21 * S21 + S[3] * S[3] + S[4] * S[4] + S31 * S31 +
                      S32 * S32 + S[5] * S[5]));
+}
+
+// 1/x and a/b rounded as by division; in FP64 without its branch where the
+// operands allow (the bounds of quot_rn, b in [2^-100, 2^120) as the 1e-30 added to
+// the coefficient's denominator leaves it)
+static __device__ __noinline__ double divided(double a, double b) { return a / b; }
+__device__ __forceinline__ float inverse_of(float x) { return 1.f / x; }
+__device__ __forceinline__ double inverse_of(double x)
+{
+    double y = rcp_rn(x);
+    if (!range_ok(x) || ones(x)) y = divided(1., x);
+    return y;
+}
+__device__ __forceinline__ float ratio_of(float a, float b) { return a / b; }
+__device__ __forceinline__ double ratio_of(double a, double b)
+{
+    double q = quot_signed(a, b, rcp_rn(b));
+    const bool in = (unsigned)(__double2hiint(b) - 0x39b00000) < 0x0dc00000u;
+    if (!in || !zero_or_range_ok(a) || ones(b)) q = divided(a, b);
+    return q;
 }
 
 template <typename T>
@@ -304,7 +328,7 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
     T Lst[6] = {};                  // Leonard stress of plane p-2
     T a1[6] = {}, a2[6] = {};       // running x sums of the filter of A
     T S1 = T(0.);                   // |S| of plane p-2
-    T t0[3] = {};                   // the y pass of plane 0
+    T t0[3] = {};                   // the y pass of plane 0 (FP32)
     double r1 = 0., r2 = 0.;        // density of planes p-1, p-2
     T x1[9] = {}, x2[9] = {};       // running x sums of the nine filters (FP32)
     if constexpr (DynSmem<T>::XS) {
@@ -326,7 +350,7 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
             if (pin && (w ? ein : in)) {
                 const int slot = w ? DYN_W * 32 + (r ? 32 : 0) + l : t;
                 const double rw = s.raw[0][slot];
-                const T rr = T(1.) / T(rw);
+                const T rr = inverse_of(T(rw));
                 v[0] = T(s.raw[1][slot]) * rr;
                 v[1] = T(s.raw[2][slot]) * rr;
                 v[2] = T(s.raw[3][slot]) * rr;
@@ -347,10 +371,13 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
         {
             const bool yp = y1 && p <= L, zp = z1 && p <= L;
             T F[9];
+            // the own row's values, formed again rather than read or kept
+            const T oq[9] = {v0[0] * h, v0[1] * h, v0[2] * h, v0[0] * v0[0] * h, v0[0] * v0[1] * h,
+                             v0[0] * v0[2] * h, v0[1] * v0[1] * h, v0[1] * v0[2] * h, v0[2] * v0[2] * h};
 #pragma unroll
             for (int m = 0; m < 9; m++) {
                 T t1 = T(0.) + s.Q[r][l][m];
-                t1 += s.Q[r + 1][l][m];
+                t1 += oq[m];
                 t1 += s.Q[r + 2][l][m];
                 if (!yp) t1 = T(0.);
                 const T th = t1 * h;
@@ -369,8 +396,14 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
                     x1[m] = T(0.) + x;
                 }
                 if (m < 3) {
-                    if (p == 1) F[m] = t0[m]; // plane 0 keeps the y pass
-                    if (p == 0) t0[m] = t1;
+                    // plane 0 keeps the y pass
+                    if constexpr (DynSmem<T>::XS) {
+                        if (p == 1) F[m] = s.t0[m][t];
+                        if (p == 0) s.t0[m][t] = t1;
+                    } else {
+                        if (p == 1) F[m] = t0[m];
+                        if (p == 0) t0[m] = t1;
+                    }
                 }
             }
             const bool none = p > L + 1 || p == 0; // nothing is written on plane L+1 (and none precedes plane 0)
@@ -383,7 +416,7 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
             Ln[3] = F[6] - F[1] * F[1]; Ln[4] = F[7] - F[1] * F[2]; Ln[5] = F[8] - F[2] * F[2];
         }
         // ---- strain rate of plane p-1: A and |S|
-        T S0 = T(0.);
+        T S0 = T(0.), oa[6];
         {
             T d[3][3], A[6];
             const T(*V)[32][3] = s.V[(p + 1) & 1];
@@ -397,7 +430,7 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
             const bool ap = z1 && p >= 2 && p <= L + 1;
             S0 = strain_of(d, A);
 #pragma unroll
-            for (int m = 0; m < 6; m++) s.A[r][l][m] = ap ? S0 * A[m] * h : T(0.);
+            for (int m = 0; m < 6; m++) s.A[r][m][l] = oa[m] = ap ? S0 * A[m] * h : T(0.);
         }
         __syncthreads();
         // ---- the filter of A, and plane p-2
@@ -406,9 +439,9 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
             T Ah[6];
 #pragma unroll
             for (int m = 0; m < 6; m++) {
-                T t1 = T(0.) + s.A[r - 1][l][m];
-                t1 += s.A[r][l][m];
-                t1 += s.A[r + 1][l][m];
+                T t1 = T(0.) + s.A[r - 1][m][l];
+                t1 += oa[m];
+                t1 += s.A[r + 1][m][l];
                 if (!y1) t1 = T(0.);
                 const T th = t1 * h;
                 T t2 = T(0.) + sh_up(th);
@@ -446,7 +479,7 @@ __global__ void __launch_bounds__(DYN_W * 32, 1)
                                 L23 * M23 + L33 * M33);
                 const T MMMM = (M11 * M11 + M12 * M12 + M13 * M13 + M12 * M12 + M22 * M22 + M23 * M23 + M13 * M13 +
                                 M23 * M23 + M33 * M33);
-                T Cd = T(-0.5) * (LLMM / (MMMM + T(1e-30)));
+                T Cd = T(-0.5) * ratio_of(LLMM, MMMM + T(1e-30));
                 if (Cd > T(0.15)) Cd = T(0.15);
                 else if (Cd < T(0.0)) Cd = T(0.0);
                 const long long c = FSL_CELL(c0 + io * g.pi, fs);
