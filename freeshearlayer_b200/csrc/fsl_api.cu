@@ -941,7 +941,7 @@ namespace fsl {
 // multi-domain stage launch (which runs the three stages, with the ghost
 // layers and boundary faces between them): the same launches fsl_step makes
 // before its first stage.
-int step_prelude32(Ctx &c)
+int step_prelude32(Ctx &c, bool ghosts)
 {
     int rc;
     if ((rc = ensure_bf(c)) || (rc = ensure_fp32(c))) return rc;
@@ -949,8 +949,8 @@ int step_prelude32(Ctx &c)
     else launch_courant(c);
     c.step++;
     draw(c);
-    if (forms_boundaries(c)) launch_ghost(c, c.U);
-    else launch_boundary32(c, c.U, c.dist);
+    if (!forms_boundaries(c)) launch_boundary32(c, c.U, c.dist);
+    else if (ghosts) launch_ghost(c, c.U);
     return step_sgs(c);
 }
 } // namespace fsl

@@ -534,11 +534,19 @@ void sequence(const Grid &g, const Consts &k, const Scratch<T> &s, const double 
     k_dyn_final<T><<<cells_grid3(b, g.L, g.H, g.D), b, 0, st>>>(g, k, U, s.Lst, s.B, s.t1, s.S, mu, cd);
 }
 
+// Planes of tiles of one evaluation.
+inline long long march_units(const Grid &g)
+{
+    return (long long)((g.D + DYN_K - 1) / DYN_K) * ((g.H + DYN_J - 1) / DYN_J) * g.L;
+}
+
 // The fused evaluation: one launch.  The march is cut so that the blocks fill
 // the SMs in whole waves: a segment of n planes costs n + 4 (the planes its
-// filters reach), and the number of waves times that is least.
+// filters reach), and the number of waves times that is least.  A domain that does
+// not have the SMs to itself is given its segments' length instead (longest 0:
+// not given).
 template <typename T>
-int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int sms, cudaStream_t st)
+int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int sms, int longest, cudaStream_t st)
 {
     static std::atomic<uint64_t> attr{0};
     if (!smem_limit_once((const void *)k_dyn_march<T>, sizeof(DynSmem<T>), attr)) return -1;
@@ -546,7 +554,11 @@ int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int
     const long long tiles = (long long)nk * nj;
     int seg = 1;
     long long best = -1;
-    for (int n = 1; n <= g.L; n++) {
+    if (longest > 0) {
+        const int segs = (g.L + longest - 1) / longest;
+        seg = (g.L + segs - 1) / segs;
+    }
+    for (int n = 1; longest <= 0 && n <= g.L; n++) {
         const long long segs = (g.L + n - 1) / n;
         if (n > 1 && segs == (g.L + n - 2) / (n - 1)) continue; // the same number of blocks with longer segments
         const long long cost = (tiles * segs + sms - 1) / sms * (n + 4);

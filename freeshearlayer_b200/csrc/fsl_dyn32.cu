@@ -10,10 +10,12 @@ FSL_CHK_EXPORT(dyn32)
 
 namespace fsl {
 
+long long dyn_units(const Grid &g) { return dyn::march_units(g); }
+
 void launch_dynsmag32(Ctx &c, const double *U, float *cd)
 {
     prof_begin(c, FSL_K_SGS);
-    dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.sms, c.stream);
+    dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.sms, c.dyn_seg, c.stream);
     prof_end(c, FSL_K_SGS, 1);
 }
 

@@ -98,12 +98,20 @@ int capture_persistent(fsl_ensemble *e, int steps)
     if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return ens_fail(e, FSL_ERR_CUDA, "cudaStreamBeginCapture");
     int rc = FSL_OK;
+    // The members' dynamic procedures run side by side: marches as long as leave the
+    // SMs about four blocks each altogether (alone, a member of 96x48x48 is cut into
+    // marches of three planes and the four its filters reach).  32 members of 48..128
+    // x 32..64 x 32..64: 2.60 -> 2.42 ms a step, the ghost passes left out below included;
+    // two to nine blocks an SM measured alike.
+    long long units = 0;
+    for (fsl_ctx *h : e->m) units += dyn_units(h->c.g);
+    for (fsl_ctx *h : e->m) h->c.dyn_seg = (int)std::max(4LL, units / (4LL * h->c.sms));
     for (int t = 0; t < steps && !rc; t++) {
         cudaEventRecord(e->cap_fork[0], e->stream);
         for (size_t q = 0; q < e->m.size(); q++) {
             Ctx &c = e->m[q]->c;
             cudaStreamWaitEvent(c.stream, e->cap_fork[0], 0);
-            if (!rc) rc = step_prelude32(c);
+            if (!rc) rc = step_prelude32(c, t == 0);
             cudaEventRecord(e->cap_join[q], c.stream);
             cudaStreamWaitEvent(e->stream, e->cap_join[q], 0);
         }
@@ -111,7 +119,10 @@ int capture_persistent(fsl_ensemble *e, int steps)
         for (fsl_ctx *h : e->m) h->c.co_valid = true;
     }
     const cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
-    for (fsl_ctx *h : e->m) h->c.step -= (unsigned)steps;
+    for (fsl_ctx *h : e->m) {
+        h->c.step -= (unsigned)steps;
+        h->c.dyn_seg = 0;
+    }
     if (rc || ce != cudaSuccess || !graph) {
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError(); // a refused capture leaves no sticky state

@@ -93,6 +93,7 @@ struct Ctx {
     float *mu32 = nullptr;
     bool fp32_alloc = false;
     int stage_tje = 0; // rows per fused-stage ring tile (incl. the two halo rows); 0: full-lane tile (FP32), by the grid (FP64)
+    int dyn_seg = 0;    // longest march of the dynamic procedure (0: as fills the SMs); set where members share them
     int stage_seg = 32; // x planes per fused-stage block (fsl_init: 48 for FP32 bulk)
     bool seg_set = false; // by fsl_tune: FP64 stages with rows 0 then run the 16-row ring tile so cut
     // learned closure
@@ -169,7 +170,9 @@ void prof_begin(Ctx &c, int cls);
 void prof_end(Ctx &c, int cls, int nkernels);
 
 int ensure_sgs(Ctx &c);          // the FP32 path's SGS field (fsl_api.cu)
-int step_prelude32(Ctx &c);      // an FP32-bulk step up to its first stage (fsl_api.cu)
+// an FP32-bulk step up to its first stage (fsl_api.cu); ghosts: U^n's ghost layer is
+// not yet written (a stage kernel that forms the boundaries leaves it written)
+int step_prelude32(Ctx &c, bool ghosts);
 int closure_step_sgs(Ctx &c);    // SGS of one step under FSL_SGS_LEARNED (fsl_closure.cu)
 int closure_ensure(Ctx &c);
 void closure_free(Ctx &c);
@@ -208,6 +211,7 @@ void launch_evolution(Ctx &c, int nstages, int stage);
 void launch_dynsmag(Ctx &c, const double *U, float *cd = nullptr); // cd: optional Cs^2 output
 // the same procedure in FP32 (the FP32-bulk path): mu_SGS into c.mu32
 void launch_dynsmag32(Ctx &c, const double *U, float *cd = nullptr);
+long long dyn_units(const Grid &g); // planes of tiles of one evaluation
 void launch_judge_rows(Ctx &c, const float *a, const float *b, double *rows);
 void launch_judge_rows(Ctx &c, const float *a, const double *b, double *rows);
 void launch_judge_rows(Ctx &c, const double *a, const double *b, double *rows);

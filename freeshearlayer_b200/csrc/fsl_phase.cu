@@ -681,7 +681,7 @@ void launch_evolution(Ctx &c, int nstages, int stage)
 void launch_dynsmag(Ctx &c, const double *U, float *cd)
 {
     prof_begin(c, FSL_K_SGS);
-    dyn::march<double>(c.g, c.k, U, c.mu, cd, c.sms, c.stream);
+    dyn::march<double>(c.g, c.k, U, c.mu, cd, c.sms, c.dyn_seg, c.stream);
     prof_end(c, FSL_K_SGS, 1);
 }
 
