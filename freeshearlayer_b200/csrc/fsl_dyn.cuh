@@ -287,6 +287,7 @@ template <typename T>
 __global__ void __launch_bounds__(DYN_W * 32, 1)
     k_dyn_march(Grid g, Consts kc, int seg, const double *__restrict__ U, T *__restrict__ mu, float *__restrict__ cd)
 {
+    follow();
     extern __shared__ __align__(16) unsigned char smraw[];
     DynSmem<T> &s = *reinterpret_cast<DynSmem<T> *>(smraw);
     const int L = g.L, H = g.H, D = g.D;
@@ -567,8 +568,8 @@ int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int
             seg = n;
         }
     }
-    k_dyn_march<T><<<dim3(nk, nj, (unsigned)((g.L + seg - 1) / seg)), DYN_W * 32, sizeof(DynSmem<T>), st>>>(g, k, seg, U,
-                                                                                                          mu, cd);
+    launch_following(k_dyn_march<T>, dim3(nk, nj, (unsigned)((g.L + seg - 1) / seg)), DYN_W * 32, sizeof(DynSmem<T>), st, g,
+                     k, seg, U, mu, cd);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

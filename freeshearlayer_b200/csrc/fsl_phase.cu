@@ -38,6 +38,7 @@ __device__ __forceinline__ long long izf(int L, int H, int D, int i, int j, int 
 // ---------------------------------------------------------------------------
 __global__ void k_ghost(Grid g, int setup, double *__restrict__ u)
 {
+    follow();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < stage::ghost_cells(g)) stage::ghost_cell(g, setup == FSL_SETUP_SPATIAL, u, t);
 }
@@ -72,6 +73,7 @@ __device__ __forceinline__ bool plane_cell(int nb, int nc, unsigned block, int &
 template <bool PPM>
 __global__ void __launch_bounds__(kPlaneThreads, 5) k_recon(Grid g, const double *__restrict__ u, Faces f)
 {
+    follow();
     const int L = g.L, H = g.H, D = g.D;
     int i, j, k;
     if (!plane_cell(H, D, blockIdx.x, i, j, k)) return;
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 5) k_recon(Grid g, const double
 // ---------------------------------------------------------------------------
 __global__ void k_ifbc(Grid g, int setup, int BL_HIG, Disturb d, Faces f)
 {
+    follow();
     const int L = g.L, H = g.H, D = g.D;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nx = (long long)H * D, ny = (long long)L * D, nz = (long long)L * H;
@@ -315,6 +318,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 5) k_flux(Grid g, Consts kc, co
                                                         const double *__restrict__ mu, Faces f, int sgs, unsigned bx,
                                                         unsigned by)
 {
+    follow();
     if (blockIdx.x < bx) flux_face<1>(g, kc, u, mu, f, sgs, blockIdx.x);
     else if (blockIdx.x < by) flux_face<2>(g, kc, u, mu, f, sgs, blockIdx.x - bx);
     else flux_face<3>(g, kc, u, mu, f, sgs, blockIdx.x - by);
@@ -328,6 +332,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 5) k_flux(Grid g, Consts kc, co
 __global__ void __launch_bounds__(kPlaneThreads) k_evolution(Grid g, int mode, const DevScalars *__restrict__ ds, double *__restrict__ U,
                             double *__restrict__ Up, Faces f)
 {
+    follow();
     const int L = g.L, H = g.H, D = g.D;
     int i, j, k;
     if (!plane_cell(H, D, blockIdx.x, i, j, k)) return;
@@ -461,6 +466,7 @@ __global__ void k_courant_to_bits(const double *__restrict__ partials, int np, D
 // accumulated over the state it wrote (that state is this step's U^n).
 __global__ void k_courant_apply(Consts kc, DevScalars *ds)
 {
+    follow();
     if (threadIdx.x == 0) apply_courant(kc, __longlong_as_double((long long)ds->co_bits), ds);
 }
 
@@ -633,7 +639,7 @@ void launch_ghost(Ctx &c, double *cur)
     const Grid &g = c.g;
     const long long n = stage::ghost_cells(g);
     prof_begin(c, FSL_K_BC);
-    k_ghost<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(g, c.k.setup, cur);
+    launch_following(k_ghost, dim3((unsigned)((n + 255) / 256)), 256, 0, c.stream, g, c.k.setup, cur);
     prof_end(c, FSL_K_BC, 1);
 }
 
@@ -642,8 +648,8 @@ void launch_recon(Ctx &c, const double *cur)
     const Grid &g = c.g;
     const unsigned n = (unsigned)g.L * plane_blocks(g.H, g.D);
     prof_begin(c, FSL_K_RECON);
-    if (c.p.recon == FSL_RECON_PPM) k_recon<true><<<n, kPlaneThreads, 0, c.stream>>>(g, cur, c.f);
-    else k_recon<false><<<n, kPlaneThreads, 0, c.stream>>>(g, cur, c.f);
+    if (c.p.recon == FSL_RECON_PPM) launch_following(k_recon<true>, dim3(n), kPlaneThreads, 0, c.stream, g, cur, c.f);
+    else launch_following(k_recon<false>, dim3(n), kPlaneThreads, 0, c.stream, g, cur, c.f);
     prof_end(c, FSL_K_RECON, 1);
 }
 
@@ -652,7 +658,7 @@ void launch_ifbc(Ctx &c, const Disturb &d)
     const Grid &g = c.g;
     const long long n = (long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H;
     prof_begin(c, FSL_K_BC);
-    k_ifbc<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(g, c.k.setup, c.k.BL_HIG, d, c.f);
+    launch_following(k_ifbc, dim3((unsigned)((n + 255) / 256)), 256, 0, c.stream, g, c.k.setup, c.k.BL_HIG, d, c.f);
     prof_end(c, FSL_K_BC, 1);
 }
 
@@ -663,7 +669,7 @@ void launch_fluxes(Ctx &c, const double *cur)
     const unsigned by = bx + (unsigned)g.L * plane_blocks(g.H + 1, g.D);
     const unsigned n = by + (unsigned)g.L * plane_blocks(g.H, g.D + 1);
     prof_begin(c, FSL_K_FLUX);
-    k_flux<<<n, kPlaneThreads, 0, c.stream>>>(g, c.k, cur, c.mu, c.f, c.p.sgs, bx, by);
+    launch_following(k_flux, dim3(n), kPlaneThreads, 0, c.stream, g, c.k, cur, c.mu, c.f, c.p.sgs, bx, by);
     prof_end(c, FSL_K_FLUX, 1);
 }
 
@@ -674,7 +680,7 @@ void launch_evolution(Ctx &c, int nstages, int stage)
     if (nstages == 2) mode = (stage == 1) ? 4 : 5;
     const unsigned n = (unsigned)g.L * plane_blocks(g.H, g.D);
     prof_begin(c, FSL_K_EVOL);
-    k_evolution<<<n, kPlaneThreads, 0, c.stream>>>(g, mode, c.ds, c.U, c.Up, c.f);
+    launch_following(k_evolution, dim3(n), kPlaneThreads, 0, c.stream, g, mode, c.ds, c.U, c.Up, c.f);
     prof_end(c, FSL_K_EVOL, 1);
 }
 
@@ -705,7 +711,7 @@ void launch_courant_to_bits(Ctx &c)
 void launch_courant_apply(Ctx &c)
 {
     prof_begin(c, FSL_K_CFL);
-    k_courant_apply<<<1, 32, 0, c.stream>>>(c.k, c.ds);
+    launch_following(k_courant_apply, dim3(1), 32, 0, c.stream, c.k, c.ds);
     prof_end(c, FSL_K_CFL, 1);
 }
 

@@ -268,6 +268,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_boundary(Grid g, int setup, int BL_HIG, Disturb d, double *__restrict__ u,
                                                   BF<T> bf)
 {
+    follow();
     const long long nf = (long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H;
     const bool spatial = setup == FSL_SETUP_SPATIAL;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -875,7 +876,7 @@ template <typename T> void launch_boundary_t(Ctx &c, double *cur, const Disturb 
     const long long n =
         2 * ((long long)g.H * g.D + (long long)g.L * g.D + (long long)g.L * g.H) + ghost_cells(g);
     prof_begin(c, FSL_K_BC);
-    k_boundary<T><<<(unsigned)((n + 127) / 128), 128, 0, c.stream>>>(g, c.k.setup, c.k.BL_HIG, d, cur, bf);
+    launch_following(k_boundary<T>, dim3((unsigned)((n + 127) / 128)), 128, 0, c.stream, g, c.k.setup, c.k.BL_HIG, d, cur, bf);
     prof_end(c, FSL_K_BC, 1);
 }
 

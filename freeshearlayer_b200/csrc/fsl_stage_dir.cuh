@@ -125,6 +125,7 @@ __device__ __forceinline__ void face_riemann(int d, const double *Lm, const doub
 template <bool SST>
 __global__ void __launch_bounds__(NT, 1) k_stage_dir(DirArgs A)
 {
+    follow();
     extern __shared__ __align__(16) unsigned char smraw[];
     Smem &s = *reinterpret_cast<Smem *>(smraw);
     typedef Kc<double> kk;
@@ -514,7 +515,7 @@ int launch_stage_dir(Ctx &c, int stage, const double *cur, const double *un, dou
     a.seg = seg;
     const unsigned tiles = (unsigned)(((c.g.D + WK - 1) / WK) * ((c.g.H + WJ - 1) / WJ));
     prof_begin(c, FSL_K_STAGE);
-    k_stage_dir<SST><<<tiles * (unsigned)((c.g.L + seg - 1) / seg), NT, sizeof(Smem), c.stream>>>(a);
+    launch_following(k_stage_dir<SST>, dim3(tiles * (unsigned)((c.g.L + seg - 1) / seg)), NT, sizeof(Smem), c.stream, a);
     prof_end(c, FSL_K_STAGE, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
