@@ -480,7 +480,7 @@ template <typename T> FSL_HD T sixth(T x)
         if (u >= 0x7e000000u || u - 1u < 0x03ffffffu) return sixth_by_division(x); // not 0 or 2^-959 .. 2^993
         constexpr double y = 1.0 / 6.0;
         const double q = __dmul_rn(x, y);
-        return __fma_rn(__fma_rn(-6.0, q, x), y, q);
+        return __fma_rn(__fma_rn(6.0, q, -x), -y, q); // (in this order -0 gives -0)
     }
 #endif
     return x / T(6.0);
