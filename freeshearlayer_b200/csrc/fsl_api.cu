@@ -871,7 +871,8 @@ int fsl_dynamic_smagorinsky(fsl_ctx *h)
     if (!h) return FSL_ERR_ARG;
     Ctx &c = h->c;
     if (c.stage_next != 0) return fail(c, FSL_ERR_ARG, "fsl_dynamic_smagorinsky: a step is in progress (fsl_step_stage)");
-    launch_dynsmag(c, c.U);
+    const int rc = launch_dynsmag(c, c.U);
+    if (rc) return rc;
     CKL();
     return FSL_OK;
 }
@@ -927,10 +928,7 @@ static int step_sgs(Ctx &c)
         if (fp32) CK(cudaMemsetAsync(c.mu32, 0, (size_t)c.g.fstride * sizeof(float), c.stream));
         else CK(cudaMemsetAsync(c.mu, 0, (size_t)c.g.fstride * sizeof(double), c.stream));
         return FSL_OK;
-    default:
-        if (fp32) launch_dynsmag32(c, c.U);
-        else launch_dynsmag(c, c.U);
-        return FSL_OK;
+    default: return fp32 ? launch_dynsmag32(c, c.U) : launch_dynsmag(c, c.U);
     }
 }
 
@@ -998,7 +996,7 @@ int fsl_step_phased(fsl_ctx *h, int nsteps)
             launch_ifbc(c, c.dist);
             if (s == 1) {
                 if (c.p.sgs == FSL_SGS_NONE) CK(cudaMemsetAsync(c.mu, 0, (size_t)c.g.fstride * sizeof(double), c.stream));
-                else if (c.p.sgs != FSL_SGS_STATIC) launch_dynsmag(c, c.U);
+                else if (c.p.sgs != FSL_SGS_STATIC && (rc = launch_dynsmag(c, c.U))) return rc;
             }
             launch_fluxes(c, cur);
             launch_evolution(c, c.p.nStages, s);

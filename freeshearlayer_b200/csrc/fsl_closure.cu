@@ -169,8 +169,8 @@ int judge_now(Ctx &c)
     const bool fp32 = c.p.precision == FSL_PREC_FP32;
     const int H = c.g.H;
     // the dynamic procedure in the path's own precision: mu into c.mu / c.mu32
-    if (fp32) launch_dynsmag32(c, c.U, c.cd32);
-    else launch_dynsmag(c, c.U, c.cd32);
+    int rc = fp32 ? launch_dynsmag32(c, c.U, c.cd32) : launch_dynsmag(c, c.U, c.cd32);
+    if (rc) return rc;
     if (launch_closure_infer(c, c.U, fp32 ? nullptr : c.mu_alt, fp32 ? c.mu32_alt : nullptr, c.cs2_32, c.cl_params,
                              c.cl_err))
         return FSL_ERR_CUDA;
@@ -181,8 +181,7 @@ int judge_now(Ctx &c)
     if (cudaMemcpyAsync(rows.data(), c.judge_rows, rows.size() * sizeof(double), cudaMemcpyDeviceToHost,
                         c.stream) != cudaSuccess)
         return FSL_ERR_CUDA;
-    int rc = check_tc_error(c);
-    if (rc) return rc;
+    if ((rc = check_tc_error(c))) return rc;
     judge_errors(rows, H, &c.last_perr, &c.last_cerr);
     std::vector<double> mrows(rows.begin() + 4 * H, rows.end());
     double mcell;
@@ -250,8 +249,8 @@ int closure_step_sgs(Ctx &c)
         return FSL_OK;
     }
     if (c.using_dynamic) {
-        if (fp32) launch_dynsmag32(c, c.U);
-        else launch_dynsmag(c, c.U);
+        const int rc = fp32 ? launch_dynsmag32(c, c.U) : launch_dynsmag(c, c.U);
+        if (rc) return rc;
         c.dynamic_steps++;
         return FSL_OK;
     }
@@ -420,7 +419,7 @@ int fsl_trainer_harvest(fsl_trainer *t, fsl_ctx *h, int stride)
     if (c.cls.DD == 0.f) return FSL_ERR_ARG; // fsl_closure_set_scales first
     if ((rc = ensure_sgs(c))) return rc;
     launch_ghost(c, c.U);
-    launch_dynsmag(c, c.U, c.cd32);
+    if ((rc = launch_dynsmag(c, c.U, c.cd32))) return rc;
     if (c.g.L < 5 || c.g.H < 5 || c.g.D < 5) return FSL_ERR_ARG;
     const long long ncell = (long long)(c.g.L - 4) * (c.g.H - 4) * (c.g.D - 4);
     const long long offset = ((long long)c.step * 7919LL) % stride;

@@ -12,11 +12,14 @@ namespace fsl {
 
 long long dyn_units(const Grid &g) { return dyn::march_units(g); }
 
-void launch_dynsmag32(Ctx &c, const double *U, float *cd)
+int launch_dynsmag32(Ctx &c, const double *U, float *cd)
 {
     prof_begin(c, FSL_K_SGS);
-    dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.sms, c.dyn_seg, c.stream);
+    const int e = dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.sms, c.dyn_seg, c.stream);
     prof_end(c, FSL_K_SGS, 1);
+    if (!e) return FSL_OK;
+    c.err = "dynamic procedure: kernel launch";
+    return FSL_ERR_CUDA;
 }
 
 } // namespace fsl

@@ -208,9 +208,10 @@ void launch_recon(Ctx &c, const double *cur);
 void launch_ifbc(Ctx &c, const Disturb &d);
 void launch_fluxes(Ctx &c, const double *cur);
 void launch_evolution(Ctx &c, int nstages, int stage);
-void launch_dynsmag(Ctx &c, const double *U, float *cd = nullptr); // cd: optional Cs^2 output
+// FSL_OK, or FSL_ERR_CUDA with c.err set; cd: optional Cs^2 output
+int launch_dynsmag(Ctx &c, const double *U, float *cd = nullptr);
 // the same procedure in FP32 (the FP32-bulk path): mu_SGS into c.mu32
-void launch_dynsmag32(Ctx &c, const double *U, float *cd = nullptr);
+int launch_dynsmag32(Ctx &c, const double *U, float *cd = nullptr);
 long long dyn_units(const Grid &g); // planes of tiles of one evaluation
 void launch_judge_rows(Ctx &c, const float *a, const float *b, double *rows);
 void launch_judge_rows(Ctx &c, const float *a, const double *b, double *rows);
