@@ -1101,20 +1101,14 @@ int fsl_step_stage(fsl_ctx *h)
     } else if (c.stage_next == 2) {
         if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step_stage: the current-stage buffer is not U^n");
         launch_boundaries(c, c.Up);
-        if (fp32) {
-            launch_stage32(c, 2, c.Up, c.U, c.Uq);
-        } else {
-            launch_stage(c, 2, c.Up, c.U, c.Uq);
-        }
+        const int e = fp32 ? launch_stage32(c, 2, c.Up, c.U, c.Uq) : launch_stage(c, 2, c.Up, c.U, c.Uq);
+        if (e) return fail(c, FSL_ERR_CUDA, "stage kernel");
         c.stage_next = 3;
     } else {
         if (c.cur != 0) return fail(c, FSL_ERR_ARG, "fsl_step_stage: the current-stage buffer is not U^n");
         launch_boundaries(c, c.Uq);
-        if (fp32) {
-            launch_stage32(c, 3, c.Uq, c.U, c.U, true);
-        } else {
-            launch_stage(c, 3, c.Uq, c.U, c.U, true);
-        }
+        const int e = fp32 ? launch_stage32(c, 3, c.Uq, c.U, c.U, true) : launch_stage(c, 3, c.Uq, c.U, c.U, true);
+        if (e) return fail(c, FSL_ERR_CUDA, "stage kernel");
         c.co_valid = true;
         c.stage_next = 0;
     }

@@ -1,6 +1,6 @@
 """A launch that the runtime refuses is reported by the call that makes it, for the
-dynamic procedure.  The refusal comes from a stand-in for the runtime's launch calls (fake_cudart.c) in
-a child process; the device sees nothing of it."""
+dynamic procedure and each stage of a step.  The refusal comes from a stand-in for the
+runtime's launch calls (fake_cudart.c) in a child process; the device sees nothing of it."""
 import pytest
 
 from tests.fake_cudart import run_child
@@ -57,3 +57,20 @@ DYNAMIC = {
 @pytest.mark.parametrize("call", DYNAMIC)
 def test_dynamic_procedure(call, prec):
     run_child(HEAD + DYNAMIC[call].format(prec=prec))
+
+# the kernels a stage can take: FP64 direction split and ring, FP32 full lane and ring
+@pytest.mark.parametrize("kernel,tune,prec", [("k_stage_dir", 0, 0), ("k_stageI", 16, 0), ("k_wide", 0, 1), ("k_stageI", 12, 1)])
+@pytest.mark.parametrize("stage", [1, 2, 3])
+def test_stages(kernel, tune, prec, stage):
+    run_child(HEAD + f"""
+d = domain(precision={prec})
+d.tune(d.TUNE_STAGE_ROWS, {tune})
+for s in (1, 2, 3):
+    if s == {stage}:
+        refused({kernel!r}, d.step_stage)
+        break
+    d.step_stage()
+d = domain(precision={prec})
+d.tune(d.TUNE_STAGE_ROWS, {tune})
+refused({kernel!r}, lambda: d.step(1), {stage - 1})
+""")
