@@ -583,7 +583,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_grad(const float *__
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     SmemTrain &s = *reinterpret_cast<SmemTrain *>(smraw);
-    if (*err) return; // an earlier pass gave up: its caller reports it
+    // an earlier pass gave up: its caller reports it.  One thread's reading for all: a
+    // block of this launch may set the flag while others start
+    if (__syncthreads_or(threadIdx.x == 0 && *err)) return;
     // cell (TMEM lane) t of the tile, columns 16 c .. 16 c + 15
     const int x = threadIdx.x, t = x & 127, c = x >> 7, wp = t >> 5, l = t & 31, c0 = c * 16;
     stage_weights(s.w, P, x, kTrainThreads);

@@ -1,0 +1,44 @@
+"""The trainer's error flag and its first state, in a child process (fake_cudart.c)
+that sets the flag as a bounded wait would and delays what the host does not wait for."""
+import pytest
+
+from tests.fake_cudart import run_child
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import numpy as np
+import freeshearlayer_b200 as fsl
+rng = np.random.default_rng(1)
+X = rng.uniform(0.1, 1.0, (1000, 8)).astype(np.float32)
+Y = rng.uniform(0.0, 0.1, 1000).astype(np.float32)
+
+def trainer():
+    t = fsl.Trainer(1024, seed=3)
+    t.set_samples(X, Y)
+    return t, fake.small()
+
+def give_up(flag):
+    one = ctypes.c_int(1)
+    assert ctypes.CDLL("libcudart.so.12").cudaMemcpy(ctypes.c_void_p(flag), ctypes.byref(one), ctypes.c_size_t(4), 1) == 0
+
+def timed_out(call):
+    try:
+        call()
+    except fsl.FslError as e:
+        return e.code == -5  # FSL_ERR_TIMEOUT
+    return False
+"""
+
+
+def test_passes_after_the_flag_do_nothing():
+    run_child(HEAD + """
+t, flag = trainer()
+w = t.weights()
+for n in (1000, 128, 1):
+    give_up(flag)
+    assert timed_out(lambda: t.gradient(n))
+give_up(flag)
+assert timed_out(lambda: t.train(2, 256))
+assert np.array_equal(t.weights(), w)
+""")
