@@ -20,7 +20,7 @@ struct fsl_trainer {
     float *X = nullptr, *Y = nullptr;      // samples
     float *P = nullptr, *M = nullptr, *V = nullptr;
     float *Gpart = nullptr, *Gout = nullptr, *lossp = nullptr;
-    int *err = nullptr;
+    int *err = nullptr; // device: the error flag, the Adam steps taken
     int maxblk = 148;
     long long adam_t = 0;
     bool shuffled = false;
@@ -384,7 +384,7 @@ int fsl_trainer_create(long long capacity, unsigned long long seed, fsl_trainer 
     ok = ok && cudaMalloc((void **)&t->Gpart, (size_t)t->maxblk * kNParams * sizeof(float)) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&t->Gout, kNParams * sizeof(float)) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&t->lossp, t->maxblk * sizeof(float)) == cudaSuccess;
-    ok = ok && cudaMalloc((void **)&t->err, sizeof(int)) == cudaSuccess;
+    ok = ok && cudaMalloc((void **)&t->err, 2 * sizeof(int)) == cudaSuccess;
     if (!ok) {
         fsl_trainer_destroy(t);
         return FSL_ERR_NOMEM;
@@ -394,7 +394,7 @@ int fsl_trainer_create(long long capacity, unsigned long long seed, fsl_trainer 
     cudaMemcpy(t->P, p.data(), kNParams * sizeof(float), cudaMemcpyHostToDevice);
     cudaMemset(t->M, 0, kNParams * sizeof(float));
     cudaMemset(t->V, 0, kNParams * sizeof(float));
-    cudaMemset(t->err, 0, sizeof(int));
+    cudaMemset(t->err, 0, 2 * sizeof(int));
     *out = t;
     return FSL_OK;
 }
@@ -483,6 +483,7 @@ int fsl_trainer_set_weights(fsl_trainer *t, const float *params)
     if (cudaMemcpyAsync(t->P, params, kNParams * sizeof(float), cudaMemcpyHostToDevice, t->st) != cudaSuccess ||
         cudaMemsetAsync(t->M, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
         cudaMemsetAsync(t->V, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->err, 0, 2 * sizeof(int), t->st) != cudaSuccess ||
         cudaStreamSynchronize(t->st) != cudaSuccess)
         return FSL_ERR_CUDA;
     t->adam_t = 0;
@@ -554,7 +555,8 @@ template <typename I> static int shuffle_samples(fsl_trainer *t)
 
 // One gradient (lr 0) or Adam pass.  With wait the host reads the loss and the
 // error flag; without, the pass is only queued: a pass that gives up sets the
-// flag, the passes after it do nothing, and the next waiting pass reports it.
+// flag, the passes after it do nothing, and the next waiting pass reports it and
+// clears it.
 static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long long n, float lr, double *loss, bool wait)
 {
     if (trainer_weights(t)) return FSL_ERR_CUDA;
@@ -581,10 +583,14 @@ static int trainer_pass(fsl_trainer *t, const float *X, const float *Y, long lon
         for (float v : lp) s += v;
         *loss = s / (double)n;
     }
-    int herr = 0;
-    cudaMemcpyAsync(&herr, t->err, sizeof(int), cudaMemcpyDeviceToHost, t->st);
+    int herr[2] = {0, 0};
+    cudaMemcpyAsync(herr, t->err, sizeof herr, cudaMemcpyDeviceToHost, t->st);
     if (cudaStreamSynchronize(t->st) != cudaSuccess) return FSL_ERR_CUDA;
-    return herr ? FSL_ERR_TIMEOUT : FSL_OK;
+    if (!herr[0]) return FSL_OK;
+    // told once; the steps that were queued but not taken don't count
+    t->adam_t = herr[1];
+    if (cudaMemsetAsync(t->err, 0, sizeof(int), t->st) != cudaSuccess) return FSL_ERR_CUDA;
+    return FSL_ERR_TIMEOUT;
 }
 
 int fsl_trainer_gradient(fsl_trainer *t, long long n, float *grad, double *loss)

@@ -255,7 +255,7 @@ void launch_harvest(Ctx &c, const float *cd, long long stride, long long offset,
 int launch_train_grad(cudaStream_t st, const float *X, const float *Y, long long n, int tpb, const float *P,
                       float *Gpart, float *loss_part, int *err, int *nblk_out, float inv_wmean);
 void launch_reduce_adam(cudaStream_t st, const float *Gpart, int nblk, float *P, float *M, float *V, float *Gout,
-                        float lr, float b1t, float b2t, const int *err);
+                        float lr, float b1t, float b2t, int *err);
 
 #ifdef __CUDACC__
 // Launch that is set up while the kernel before it on the stream still runs (its

@@ -820,12 +820,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_grad(const float *__
 }
 
 // Deterministic sum of the block partials and an Adam step (FP32 master
-// weights); no step after a pass that gave up.  The partials are read eight
+// weights), counted in err[1]; no step after a pass that gave up.  The partials are read eight
 // at a time (a serial chain of loads per parameter otherwise) and added in
 // block order.
 __global__ void k_reduce_adam(const float *__restrict__ Gpart, int nblk, float *__restrict__ P,
                               float *__restrict__ Mo, float *__restrict__ Vo, float *__restrict__ Gout, float lr,
-                              float b1t, float b2t, const int *err)
+                              float b1t, float b2t, int *err)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kNParams || *err) return;
@@ -839,6 +839,7 @@ __global__ void k_reduce_adam(const float *__restrict__ Gpart, int nblk, float *
     }
     if (Gout) Gout[p] = g;
     if (lr <= 0.f) return;
+    if (p == 0) err[1]++;
     const bool padded = (p >= kOffW1 && p < kOffW1 + 64 * 16 && ((p - kOffW1) % 16) >= 8);
     if (padded) return;
     const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
@@ -929,7 +930,7 @@ int launch_train_grad(cudaStream_t st, const float *X, const float *Y, long long
 }
 
 void launch_reduce_adam(cudaStream_t st, const float *Gpart, int nblk, float *P, float *M, float *V, float *Gout,
-                        float lr, float b1t, float b2t, const int *err)
+                        float lr, float b1t, float b2t, int *err)
 {
     mlp::k_reduce_adam<<<(kNParams + 63) / 64, 64, 0, st>>>(Gpart, nblk, P, M, V, Gout, lr, b1t, b2t, err);
 }

@@ -42,3 +42,24 @@ give_up(flag)
 assert timed_out(lambda: t.train(2, 256))
 assert np.array_equal(t.weights(), w)
 """)
+
+
+@pytest.mark.parametrize("first", ["train", "gradient", "set_weights"])
+def test_a_reported_flag_is_cleared_and_its_steps_not_counted(first):
+    run_child(HEAD + f"""
+t, flag = trainer()
+t.train(2, 256)
+give_up(flag)
+if {first!r} == "set_weights":
+    t.set_weights(t.weights())
+else:
+    assert timed_out(lambda: t.train(3, 256) if {first!r} == "train" else t.gradient())
+u, _ = trainer()
+u.train(2, 256)
+if {first!r} == "set_weights":
+    u.set_weights(u.weights())
+a, b = t.gradient(), u.gradient()
+assert a[1] == b[1] and np.array_equal(a[0], b[0])
+assert t.train(2, 256) == u.train(2, 256)  # the same Adam step count, too
+assert np.array_equal(t.weights(), u.weights())
+""")
