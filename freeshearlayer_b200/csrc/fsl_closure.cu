@@ -391,10 +391,15 @@ int fsl_trainer_create(long long capacity, unsigned long long seed, fsl_trainer 
     }
     std::vector<float> p;
     init_params(p, seed);
-    cudaMemcpy(t->P, p.data(), kNParams * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemset(t->M, 0, kNParams * sizeof(float));
-    cudaMemset(t->V, 0, kNParams * sizeof(float));
-    cudaMemset(t->err, 0, 2 * sizeof(int));
+    // on the trainer's own stream, which the passes queued on it follow
+    if (cudaMemcpyAsync(t->P, p.data(), kNParams * sizeof(float), cudaMemcpyHostToDevice, t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->M, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->V, 0, kNParams * sizeof(float), t->st) != cudaSuccess ||
+        cudaMemsetAsync(t->err, 0, 2 * sizeof(int), t->st) != cudaSuccess ||
+        cudaStreamSynchronize(t->st) != cudaSuccess) {
+        fsl_trainer_destroy(t);
+        return FSL_ERR_CUDA;
+    }
     *out = t;
     return FSL_OK;
 }

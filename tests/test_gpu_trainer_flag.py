@@ -63,3 +63,14 @@ assert a[1] == b[1] and np.array_equal(a[0], b[0])
 assert t.train(2, 256) == u.train(2, 256)  # the same Adam step count, too
 assert np.array_equal(t.weights(), u.weights())
 """)
+
+
+def test_a_new_trainer_waits_for_its_first_state():
+    run_child(HEAD + """
+u, _ = trainer()
+fake.late(True)
+t, _ = trainer()
+a = t.train(2, 256)
+fake.late(False)
+assert a == u.train(2, 256) and np.array_equal(t.weights(), u.weights())
+""")
