@@ -219,6 +219,11 @@ void launch_judge_rows(Ctx &c, const double *a, const double *b, double *rows);
 void launch_courant(Ctx &c);
 // dt update from the Courant maximum the fused stage 3 accumulated
 void launch_courant_apply(Ctx &c);
+// Planes of HIG x 5 rows that one launch of the row kernels moves: their 32-bit row
+// numbers, the step past the last included, stay below 2^32 (a plane of a domain
+// of 2^31 cells has at most 5 x 2^29 rows).
+constexpr unsigned kRowBlocks = 148 * 8;
+inline long long rows_batch(int H) { return (0xffffffffLL - 8 * kRowBlocks) / (5LL * H); }
 void launch_state_scatter(Ctx &c, double *dst, const double *packed, int i0, int ni);
 void launch_state_gather(Ctx &c, const double *src, double *packed, int i0, int ni);
 void launch_courant_to_bits(Ctx &c);

@@ -722,13 +722,18 @@ template <bool GATHER> static void state_rows(Ctx &c, double *fields, double *pa
 {
     if (ni <= 0) return;
     const Grid &g = c.g;
-    const unsigned nrows = (unsigned)((long long)ni * g.H * 5); // at most 2^31 cells of DEP >= 2
-    const unsigned nblk = std::min((nrows + 7u) / 8u, 148u * 8u);
+    const long long batch = rows_batch(g.H);
     prof_begin(c, FSL_K_OTHER);
-    if (g.D % 2 == 0 && (uintptr_t)packed % 16 == 0)
-        k_state_rows<GATHER, double2><<<nblk, 256, 0, c.stream>>>(g, fields, packed, i0, nrows);
-    else k_state_rows<GATHER, double><<<nblk, 256, 0, c.stream>>>(g, fields, packed, i0, nrows);
-    prof_end(c, FSL_K_OTHER, 1);
+    int launches = 0;
+    for (long long b = 0; b < ni; b += batch, launches++) {
+        const unsigned nrows = (unsigned)(std::min(batch, ni - b) * g.H * 5);
+        const unsigned nblk = std::min((nrows + 7u) / 8u, kRowBlocks);
+        double *p = packed + b * g.H * 5 * g.D;
+        if (g.D % 2 == 0 && (uintptr_t)p % 16 == 0)
+            k_state_rows<GATHER, double2><<<nblk, 256, 0, c.stream>>>(g, fields, p, i0 + (int)b, nrows);
+        else k_state_rows<GATHER, double><<<nblk, 256, 0, c.stream>>>(g, fields, p, i0 + (int)b, nrows);
+    }
+    prof_end(c, FSL_K_OTHER, launches);
 }
 
 void launch_state_scatter(Ctx &c, double *dst, const double *packed, int i0, int ni)
