@@ -1,0 +1,45 @@
+"""Which FP64 stage kernel runs, counted in a child process (fake_cudart.c): the grid's
+choice, the tuning calls that set it aside and bring it back, and the ensembles
+that capture it."""
+import pytest
+
+from tests.fake_cudart import run_child
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import time
+import numpy as np
+import freeshearlayer_b200 as fsl
+from tests.helpers import random_state, spatial_params, temporal_params
+
+DIR, RING = "k_stage_dir", "k_stageI"
+
+def domain(L, H, D, setup="temporal", **kw):
+    p = temporal_params(L, H, D, deltaT=1e-6, **kw) if setup == "temporal" else spatial_params(L, H, D)
+    d = fsl.Domain(p)
+    d.upload_state(random_state(p, 11))
+    return d, p
+
+def ran(call):
+    fake.reset()
+    call()
+    return fake.count(DIR), fake.count(RING)
+"""
+
+
+# grids on either side of the rule (148 SMs); the ring in both setups, its last
+# segment and its last tiles ragged
+@pytest.mark.parametrize("L,H,D,setup,ring", [(64, 32, 32, "temporal", False), (37, 56, 30, "temporal", True),
+                                              (77, 27, 57, "temporal", True), (40, 30, 30, "spatial", True)])
+def test_the_grids_choice_equals_oracle(L, H, D, setup, ring):
+    run_child(HEAD + f"""
+from oracle import oracle as orc
+orc.build()
+d, p = domain({L}, {H}, {D}, {setup!r})
+assert ran(lambda: d.step(2)) == ((0, 6) if {ring} else (6, 0))
+o = orc.Oracle(p)
+o.set_state(random_state(p, 11))
+o.step(2)
+assert np.all(np.isfinite(o.state())) and np.array_equal(d.download_state(), o.state())
+""")
