@@ -310,6 +310,7 @@ static void check_shapes(fsl_ensemble *e)
     for (fsl_ctx *h : e->m) {
         sig.push_back(h->c.stage_tje);
         sig.push_back(h->c.stage_seg);
+        sig.push_back(h->c.seg_set);
     }
     if (sig != e->sig) {
         e->sig = sig;

@@ -43,3 +43,18 @@ o.set_state(random_state(p, 11))
 o.step(2)
 assert np.all(np.isfinite(o.state())) and np.array_equal(d.download_state(), o.state())
 """)
+
+
+def test_ensemble_captures_again_after_tuning_a_member():
+    run_child(HEAD + """
+d, _ = domain(64, 32, 32)
+e = fsl.Ensemble([d])
+e.set_chunk(2)
+e.step(5)
+fake.reset()
+e.step(4)
+assert fake.graphs() == 0
+d.tune(d.TUNE_STAGE_SEG, 32)  # the value it has by default
+assert ran(lambda: e.step(4)) == (0, 6) and fake.graphs() == 1
+e.sync()
+""")
