@@ -400,9 +400,11 @@ int fsl_ensemble_tune(fsl_ensemble *e, int trial_steps, int *rows_out, int *seg_
     for (size_t q = 0; q < e->m.size(); q++)
         if ((rc = take(e->m[q]->c, snap[q]))) return ens_fail(e, rc, "tuner snapshot");
     // rows 0: the full-lane persistent tile (FP32 bulk, reference scheme;
-    // it balances its own planes, so one planes-per-block value is tried)
+    // it balances its own planes, so one planes-per-block value is tried) or the kernel
+    // and the planes per block the grid calls for (FP64)
     const int rows_c[4] = {0, 8, 12, 16}, seg_c[5] = {8, 16, 32, 48, 64};
     int best_r = e->m[0]->c.stage_tje, best_s = e->m[0]->c.stage_seg;
+    bool best_set = e->m[0]->c.seg_set;
     double best = 1e300;
     cudaEvent_t a = nullptr, b = nullptr;
     cudaEventCreate(&a);
@@ -412,6 +414,7 @@ int fsl_ensemble_tune(fsl_ensemble *e, int trial_steps, int *rows_out, int *seg_
             for (fsl_ctx *h : e->m) {
                 h->c.stage_tje = rows_c[ri];
                 h->c.stage_seg = seg_c[si];
+                h->c.seg_set = rows_c[ri] != 0;
             }
             e->gen++;
             // one plain step per member (sets the kernels' attributes outside
@@ -435,6 +438,7 @@ int fsl_ensemble_tune(fsl_ensemble *e, int trial_steps, int *rows_out, int *seg_
                 best = per;
                 best_r = rows_c[ri];
                 best_s = seg_c[si];
+                best_set = rows_c[ri] != 0;
             }
         }
     cudaEventDestroy(a);
@@ -445,6 +449,7 @@ int fsl_ensemble_tune(fsl_ensemble *e, int trial_steps, int *rows_out, int *seg_
         Ctx &c = e->m[q]->c;
         c.stage_tje = best_r;
         c.stage_seg = best_s;
+        c.seg_set = best_set;
         const int r2 = restore(c, snap[q]);
         if (!rc) rc = r2;
         cudaFree(snap[q].U);

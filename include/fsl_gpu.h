@@ -526,7 +526,9 @@ int fsl_ensemble_set_barrier_limit(fsl_ensemble *e, unsigned polls);
  * block 8/16/32/64, one shape for all members): each candidate is timed on
  * the device over one graph replay of trial_steps ensemble steps; the
  * fastest is kept and every member's state, time step and counters are
- * restored, so tuning changes no result. */
+ * restored, so tuning changes no result.  *rows 0: FP64 members run the kernel and
+ * the planes per block their grids call for, whatever *seg says (setting it with
+ * fsl_tune would take them off it). */
 int fsl_ensemble_tune(fsl_ensemble *ens, int trial_steps, int *rows, int *seg, double *ms_per_step);
 
 /* ---- profiling ------------------------------------------------------------- */

@@ -58,3 +58,16 @@ d.tune(d.TUNE_STAGE_SEG, 32)  # the value it has by default
 assert ran(lambda: e.step(4)) == (0, 6) and fake.graphs() == 1
 e.sync()
 """)
+
+
+def test_ensemble_tuner_measures_the_grids_choice():
+    run_child(HEAD + """
+d, _ = domain(64, 32, 32)
+d.tune(d.TUNE_STAGE_SEG, 20)
+e = fsl.Ensemble([d])
+fake.reset()
+rows, seg, _ = e.tune(trial_steps=2)
+assert fake.count(DIR) == 9  # one plain step and one captured chunk of two
+assert ran(lambda: d.step(1)) == ((3, 0) if rows == 0 else (0, 3))
+e.sync()
+""")
