@@ -1150,6 +1150,7 @@ int fsl_tune(fsl_ctx *h, int key, int value)
     case FSL_TUNE_STAGE_ROWS:
         if (value != 0 && value != 8 && value != 12 && value != 16) return FSL_ERR_ARG;
         c.stage_tje = value;
+        if (value == 0) c.seg_set = false; // back to what the grid calls for
         return FSL_OK;
     case FSL_TUNE_STAGE_SEG:
         if (value < 1 || value > 1 << 20) return FSL_ERR_ARG;

@@ -309,7 +309,8 @@ int fsl_step_stage(fsl_ctx *ctx);
 #define FSL_TUNE_STAGE_ROWS 1 /* rows per ring stage tile incl. 2 halo rows: 8, 12 or 16; or 0, the
                                  default: the full-lane persistent 16 x 32 tile (FP32 bulk with the
                                  reference reconstruction), 16 (FP32 bulk with PPM), or the kernel and
-                                 the planes per block the grid calls for (FP64) */
+                                 the planes per block the grid calls for (FP64: also after
+                                 FSL_TUNE_STAGE_SEG, which a later 0 here sets aside) */
 #define FSL_TUNE_STAGE_SEG 2  /* x planes marched per ring-tile stage block (default 48 FP32 bulk, 32 FP64;
                                  with rows 0 the FP32 bulk's full-lane tile splits the planes itself, FP64
                                  stages run 16 rows once this is set) */

@@ -71,3 +71,17 @@ assert fake.count(DIR) == 9  # one plain step and one captured chunk of two
 assert ran(lambda: d.step(1)) == ((3, 0) if rows == 0 else (0, 3))
 e.sync()
 """)
+
+
+def test_rows_zero_returns_to_the_grids_choice():
+    run_child(HEAD + """
+d, _ = domain(64, 32, 32)
+assert ran(lambda: d.step(1)) == (3, 0)
+d.tune(d.TUNE_STAGE_SEG, 16)
+assert ran(lambda: d.step(1)) == (0, 3)
+d.tune(d.TUNE_STAGE_ROWS, 0)
+assert ran(lambda: d.step(1)) == (3, 0)
+d.tune(d.TUNE_STAGE_ROWS, 0)
+d.tune(d.TUNE_STAGE_SEG, 16)
+assert ran(lambda: d.step(1)) == (0, 3)
+""")
