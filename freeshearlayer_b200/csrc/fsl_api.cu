@@ -415,6 +415,8 @@ int fsl_init(const fsl_params *p, fsl_ctx **out)
     // persistent tile, FP32 PPM stages the 16-row ring tile; FP64 stages pick
     // their kernel and split by the grid (fsl_fused.cu)
     c.stage_tje = 0;
+    stage_cuts(c);
+    c.dyn_cut = dyn_cut(c.g, c.sms);
     // derived constants, src/initialize.c:67-94
     c.k.rdx = 1. / p->deltaX; c.k.rdy = 1. / p->deltaY; c.k.rdz = 1. / p->deltaZ;
     c.k.r4dx = 1. / (4 * p->deltaX); c.k.r4dy = 1. / (4 * p->deltaY); c.k.r4dz = 1. / (4 * p->deltaZ);

@@ -541,25 +541,15 @@ inline long long march_units(const Grid &g)
     return (long long)((g.D + DYN_K - 1) / DYN_K) * ((g.H + DYN_J - 1) / DYN_J) * g.L;
 }
 
-// The fused evaluation: one launch.  The march is cut so that the blocks fill
+// The march is cut so that the blocks fill
 // the SMs in whole waves: a segment of n planes costs n + 4 (the planes its
-// filters reach), and the number of waves times that is least.  A domain that does
-// not have the SMs to itself is given its segments' length instead (longest 0:
-// not given).
-template <typename T>
-int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int sms, int longest, cudaStream_t st)
+// filters reach), and the number of waves times that is least.
+inline int march_cut(const Grid &g, int sms)
 {
-    static std::atomic<uint64_t> attr{0};
-    if (!smem_limit_once((const void *)k_dyn_march<T>, sizeof(DynSmem<T>), attr)) return -1;
-    const unsigned nk = (unsigned)((g.D + DYN_K - 1) / DYN_K), nj = (unsigned)((g.H + DYN_J - 1) / DYN_J);
-    const long long tiles = (long long)nk * nj;
+    const long long tiles = march_units(g) / g.L;
     int seg = 1;
     long long best = -1;
-    if (longest > 0) {
-        const int segs = (g.L + longest - 1) / longest;
-        seg = (g.L + segs - 1) / segs;
-    }
-    for (int n = 1; longest <= 0 && n <= g.L; n++) {
+    for (int n = 1; n <= g.L; n++) {
         const long long segs = (g.L + n - 1) / n;
         if (n > 1 && segs == (g.L + n - 2) / (n - 1)) continue; // the same number of blocks with longer segments
         const long long cost = (tiles * segs + sms - 1) / sms * (n + 4);
@@ -567,6 +557,23 @@ int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int
             best = cost;
             seg = n;
         }
+    }
+    return seg;
+}
+
+// The fused evaluation: one launch, marches of `cut` planes.  A domain that does
+// not have the SMs to itself is given the length of its longest march instead, which
+// its marches share evenly (longest 0: not given).
+template <typename T>
+int march(const Grid &g, const Consts &k, const double *U, T *mu, float *cd, int cut, int longest, cudaStream_t st)
+{
+    static std::atomic<uint64_t> attr{0};
+    if (!smem_limit_once((const void *)k_dyn_march<T>, sizeof(DynSmem<T>), attr)) return -1;
+    const unsigned nk = (unsigned)((g.D + DYN_K - 1) / DYN_K), nj = (unsigned)((g.H + DYN_J - 1) / DYN_J);
+    int seg = cut;
+    if (longest > 0) {
+        const int segs = (g.L + longest - 1) / longest;
+        seg = (g.L + segs - 1) / segs;
     }
     launch_following(k_dyn_march<T>, dim3(nk, nj, (unsigned)((g.L + seg - 1) / seg)), DYN_W * 32, sizeof(DynSmem<T>), st, g,
                      k, seg, U, mu, cd);

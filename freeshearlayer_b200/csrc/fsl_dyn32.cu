@@ -11,11 +11,12 @@ FSL_CHK_EXPORT(dyn32)
 namespace fsl {
 
 long long dyn_units(const Grid &g) { return dyn::march_units(g); }
+int dyn_cut(const Grid &g, int sms) { return dyn::march_cut(g, sms); }
 
 int launch_dynsmag32(Ctx &c, const double *U, float *cd)
 {
     prof_begin(c, FSL_K_SGS);
-    const int e = dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.sms, c.dyn_seg, c.stream);
+    const int e = dyn::march<float>(c.g, c.k, U, c.mu32, cd, c.dyn_cut, c.dyn_seg, c.stream);
     prof_end(c, FSL_K_SGS, 1);
     if (!e) return FSL_OK;
     c.err = "dynamic procedure: kernel launch";

@@ -23,11 +23,8 @@ void launch_boundary(Ctx &c, double *cur, const Disturb &d)
 
 // How a domain's tiles (tj x tk output cells) are cut along x when one block
 // fits on an SM: the blocks run in waves and a segment of n planes costs n +
-// `start` planes, so take the n whose waves cost least.
-struct Cut {
-    int seg;     // planes per block
-    double cost; // planes one SM marches, starts included
-};
+// `start` planes, so take the n whose waves cost least.  One search over all n a domain
+// (2.6 ms at 2^20 planes), not one a launch.
 static Cut cut_tiles(const Grid &g, int sms, int tj, int tk, double start)
 {
     const long long tiles = (long long)((g.D + tk - 1) / tk) * ((g.H + tj - 1) / tj);
@@ -39,8 +36,12 @@ static Cut cut_tiles(const Grid &g, int sms, int tj, int tk, double start)
     }
     return best;
 }
-static Cut ring_cut(const Grid &g, int sms, int tj) { return cut_tiles(g, sms, tj, 30, 1.2); }
-static Cut dir_cut(const Grid &g, int sms) { return cut_tiles(g, sms, dirs::WJ, dirs::WK, 2.0); }
+void stage_cuts(Ctx &c)
+{
+    c.ring_cut = cut_tiles(c.g, c.sms, 14, 30, 1.2);
+    c.ppm_cut = cut_tiles(c.g, c.sms, 10, 30, 1.2);
+    c.dir_cut = cut_tiles(c.g, c.sms, dirs::WJ, dirs::WK, 2.0);
+}
 
 // The ring tile marches a plane of 14 x 30 cells in 10.8 us, the direction-split
 // kernel one of 4 x 32 in 4.95 us and 3 us a launch, whatever the grid (measured
@@ -54,7 +55,7 @@ bool stage_splits_directions(const Ctx &c)
 {
     if (c.p.recon != FSL_RECON_CHARMINMOD || c.stage_tje != 0 || c.seg_set) return false;
     const double pass = c.p.setup == FSL_SETUP_TEMPORAL ? 6. : 0.;
-    return 3. + 4.95 * dir_cut(c.g, c.sms).cost < 10.8 * ring_cut(c.g, c.sms, 14).cost + pass;
+    return 3. + 4.95 * c.dir_cut.cost < 10.8 * c.ring_cut.cost + pass;
 }
 
 template <bool SST>
@@ -67,14 +68,14 @@ static int stage64(Ctx &c, int stage, const double *cur, const double *un, doubl
         if (c.stage_tje == 8)
             return stage::launch_stage_t<double, 8, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
         return stage::launch_stage_t<double, 12, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant,
-                                                               c.stage_tje || c.seg_set ? 0 : ring_cut(c.g, c.sms, 10).seg);
+                                                               c.stage_tje || c.seg_set ? 0 : c.ppm_cut.seg);
     }
     switch (c.stage_tje) {
     case 0:
         if (stage_splits_directions(c))
-            return dirs::launch_stage_dir<SST>(c, stage, cur, un, out, c.mu, bf64(c), courant, dir_cut(c.g, c.sms).seg);
+            return dirs::launch_stage_dir<SST>(c, stage, cur, un, out, c.mu, bf64(c), courant, c.dir_cut.seg);
         return stage::launch_stage_t<double, 16, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant,
-                                                                c.seg_set ? 0 : ring_cut(c.g, c.sms, 14).seg);
+                                                                c.seg_set ? 0 : c.ring_cut.seg);
     case 8: return stage::launch_stage_t<double, 8, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
     case 12: return stage::launch_stage_t<double, 12, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);
     default: return stage::launch_stage_t<double, 16, 1, false, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);

@@ -74,6 +74,12 @@ struct BFaces32 {
     float *x0, *xL, *y0, *yH, *z0, *zD;
 };
 
+// How a domain's tiles are cut along x (fsl_fused.cu).
+struct Cut {
+    int seg;     // planes per block
+    double cost; // planes one SM marches, starts included
+};
+
 struct Ctx {
     fsl_params p;
     Consts k;
@@ -93,7 +99,11 @@ struct Ctx {
     float *mu32 = nullptr;
     bool fp32_alloc = false;
     int stage_tje = 0; // rows per fused-stage ring tile (incl. the two halo rows); 0: full-lane tile (FP32), by the grid (FP64)
-    int dyn_seg = 0;    // longest march of the dynamic procedure (0: as fills the SMs); set where members share them
+    // the cuts the grid calls for, found once (fsl_init): the FP64 ring, its PPM tile, the
+    // direction split; planes per march of the dynamic procedure
+    Cut ring_cut{}, ppm_cut{}, dir_cut{};
+    int dyn_cut = 1;
+    int dyn_seg = 0;    // longest march of the dynamic procedure (0: dyn_cut); set where members share the SMs
     int stage_seg = 32; // x planes per fused-stage block (fsl_init: 48 for FP32 bulk)
     bool seg_set = false; // by fsl_tune: FP64 stages with rows 0 then run the 16-row ring tile so cut
     // learned closure
@@ -213,6 +223,7 @@ int launch_dynsmag(Ctx &c, const double *U, float *cd = nullptr);
 // the same procedure in FP32 (the FP32-bulk path): mu_SGS into c.mu32
 int launch_dynsmag32(Ctx &c, const double *U, float *cd = nullptr);
 long long dyn_units(const Grid &g); // planes of tiles of one evaluation
+int dyn_cut(const Grid &g, int sms); // planes per march of a domain alone
 void launch_judge_rows(Ctx &c, const float *a, const float *b, double *rows);
 void launch_judge_rows(Ctx &c, const float *a, const double *b, double *rows);
 void launch_judge_rows(Ctx &c, const double *a, const double *b, double *rows);
@@ -235,6 +246,7 @@ void launch_plane_sums(Ctx &c, const double *U, int i0, int ni, double *rows);
 void launch_boundary(Ctx &c, double *cur, const Disturb &d);
 // One RK3 stage: cur (ghosts filled) -> out; un = U^n.
 int launch_stage(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant = false);
+void stage_cuts(Ctx &c); // c.ring_cut, c.ppm_cut, c.dir_cut
 // whether launch_stage runs the direction-split kernel (rows 0, small grids)
 bool stage_splits_directions(const Ctx &c);
 // FP32-bulk variants (fsl_fused32.cu): boundary states in bf32, SGS viscosity in mu32.

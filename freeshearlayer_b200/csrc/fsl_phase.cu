@@ -687,7 +687,7 @@ void launch_evolution(Ctx &c, int nstages, int stage)
 int launch_dynsmag(Ctx &c, const double *U, float *cd)
 {
     prof_begin(c, FSL_K_SGS);
-    const int e = dyn::march<double>(c.g, c.k, U, c.mu, cd, c.sms, c.dyn_seg, c.stream);
+    const int e = dyn::march<double>(c.g, c.k, U, c.mu, cd, c.dyn_cut, c.dyn_seg, c.stream);
     prof_end(c, FSL_K_SGS, 1);
     if (!e) return FSL_OK;
     c.err = "dynamic procedure: kernel launch";

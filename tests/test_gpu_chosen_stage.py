@@ -85,3 +85,20 @@ d.tune(d.TUNE_STAGE_ROWS, 0)
 d.tune(d.TUNE_STAGE_SEG, 16)
 assert ran(lambda: d.step(1)) == (0, 3)
 """)
+
+
+def test_a_long_domains_launches_cost_the_host_little():
+    # 2^20 planes: a search over every segment length takes milliseconds, and a step
+    # needs a dozen of its results
+    run_child(HEAD + """
+d, _ = domain(1 << 20, 2, 2, deltaX=1.0, deltaY=1.0, deltaZ=1.0)
+d.step(1)
+d.sync()
+best = 1e9
+for _ in range(3):
+    t0 = time.perf_counter()
+    d.step(1)
+    best = min(best, time.perf_counter() - t0)
+    d.sync()
+assert best < 5e-3, best
+""")
