@@ -128,17 +128,10 @@ __device__ __forceinline__ double quot_signed(double a, double b, double y)
 }
 // positive and in [2^-60, 2^60)
 __device__ __forceinline__ bool range_ok(double x) { return (unsigned)(__double2hiint(x) - 0x3c300000) < 0x07800000u; }
-// the magnitude's high word, odd where the low word is not zero: a subnormal whose
-// high word is zero is not taken for zero
-__device__ __forceinline__ unsigned magnitude(double x)
-{
-    return ((unsigned)__double2hiint(x) & 0x7fffffffu) | min((unsigned)__double2loint(x), 1u);
-}
-// zero, or of magnitude in [2^-512, 2^120)
+// zero, or of magnitude in [2^-512, 2^120) (the high word twice drops the sign)
 __device__ __forceinline__ bool zero_or_range_ok(double x)
 {
-    const unsigned u = magnitude(x);
-    return u < 0x47700000u && u - 1u >= 0x1fefffffu;
+    return 2u * (unsigned)__double2hiint(x) - 0x3fe00000u < 0x4f000000u || x == 0.0;
 }
 // a significand whose low word is all ones
 __device__ __forceinline__ bool ones(double x) { return __double2loint(x) == -1; }
@@ -476,8 +469,8 @@ template <typename T> FSL_HD T sixth(T x)
 {
 #ifdef __CUDA_ARCH__
     if constexpr (std::is_same<T, double>::value) {
-        const unsigned u = magnitude(x);
-        if (u >= 0x7e000000u || u - 1u < 0x03ffffffu) return sixth_by_division(x); // not 0 or 2^-959 .. 2^993
+        // not of magnitude in [2^-959, 2^993), nor zero
+        if (2u * (unsigned)__double2hiint(x) - 0x08000000u >= 0xf4000000u && x != 0.0) return sixth_by_division(x);
         constexpr double y = 1.0 / 6.0;
         const double q = __dmul_rn(x, y);
         return __fma_rn(__fma_rn(6.0, q, -x), -y, q); // (in this order -0 gives -0)
