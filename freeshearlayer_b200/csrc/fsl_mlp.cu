@@ -583,9 +583,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_grad(const float *__
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     SmemTrain &s = *reinterpret_cast<SmemTrain *>(smraw);
-    // an earlier pass gave up: its caller reports it.  One thread's reading for all: a
-    // block of this launch may set the flag while others start
-    if (__syncthreads_or(threadIdx.x == 0 && *err)) return;
+    const int gave_up = threadIdx.x == 0 ? *err : 0; // in flight while the weights are staged
     // cell (TMEM lane) t of the tile, columns 16 c .. 16 c + 15
     const int x = threadIdx.x, t = x & 127, c = x >> 7, wp = t >> 5, l = t & 31, c0 = c * 16;
     stage_weights(s.w, P, x, kTrainThreads);
@@ -599,6 +597,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_grad(const float *__
     for (int e = x; e < 128 * 16; e += kTrainThreads) s.A0[e] = s.A0T[e] = __float2bfloat16_rn(0.f);
     if (x == 0) umma::mbar_init(&s.mbar, 1);
     float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, gw4 = 0.f, gb4 = 0.f, loss = 0.f;
+    // an earlier pass gave up: its caller reports it.  One thread's reading for all: a
+    // block of this launch may set the flag while others start
+    if (__syncthreads_or(gave_up)) return;
     if (x < 32) umma::tmem_alloc(&s.tholder, 512);
     umma::fence_before_sync();
     __syncthreads();
