@@ -61,9 +61,10 @@ bool stage_splits_directions(const Ctx &c)
 template <bool SST>
 static int stage64(Ctx &c, int stage, const double *cur, const double *un, double *out, bool courant)
 {
-    // PPM: halo 2, a ring of four planes.  A 16-row FP64 tile would need more
-    // than the 227 KB of shared memory a block may have; 12 rows measured
-    // fastest at 512x256x256 (54 ms per step against 69 for 8), so 16 runs as 12
+    // PPM: halo 2, a ring of five planes, the one in flight included.  A 16-row FP64
+    // tile would need more than the 227 KB of shared memory a block may have; 12 rows
+    // measured fastest at 512x256x256 (35.5 ms per step against 46.4 for 8, and 34.5 with
+    // the planes per block by the grid), so 16 runs as 12
     if (c.p.recon == FSL_RECON_PPM) {
         if (c.stage_tje == 8)
             return stage::launch_stage_t<double, 8, 1, true, SST>(c, stage, cur, un, out, c.mu, bf64(c), courant);

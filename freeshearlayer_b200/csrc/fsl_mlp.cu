@@ -569,7 +569,7 @@ __device__ __forceinline__ float warp_colsum16(const float *in, int l)
 // accumulated per block into Gpart[blockIdx.x][kNParams]; loss_part holds
 // the block's summed squared error.  Each block handles tiles
 // [blockIdx.x * tpb, (blockIdx.x + 1) * tpb).  TMEM (448 of 512 columns) allows
-// one block per SM, so the chain of seven products and their epilogues bounds
+// one block per SM, so the chain of six waits for eight products and their epilogues bounds
 // it; four threads share a cell (a TMEM lane), each with 16 of a layer's 64
 // columns, so that four warps a scheduler hide the epilogues' latency (a
 // gradient of 2^20 samples: 0.85 ms with one thread a cell, 0.51 ms now).  The bias,

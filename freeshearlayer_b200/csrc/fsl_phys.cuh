@@ -46,8 +46,9 @@ template <typename T> FSL_HD T minmod(T x, T y)
 
 // minmod(a, b) and minmod(b, a) at once: both are 0 when a b <= 0, else
 // sign(a) min(|a|, 4|b|) and sign(b) min(|b|, 4|a|) -- exactly the values of
-// the select form above (min, |.|, x4 and the sign copy are exact), with one
-// product and one sign test for the pair.  FP64 takes the minimum as a compare
+// the select form above (min, |.|, x4 and the sign copy are exact; in FP64, where one
+// of the two is NaN, so is one result in either form, and the sweep adds the two), with
+// one product and one sign test for the pair.  FP64 takes the minimum as a compare
 // and a select and the sign by bits, which keeps the FP64 pipe to six
 // instructions a pair instead of fourteen (with the stored roots of the ring
 // tile, stage::Smem::C, the FP64 stage went from 8.35 to 7.30 ms a launch at

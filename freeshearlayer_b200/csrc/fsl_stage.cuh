@@ -13,9 +13,10 @@
 // the face-averaged SGS viscosity.  Every face flux of the tile is computed
 // once (x faces in registers carried along the march, y faces through shared
 // memory, z faces through warp shuffles); the state is read once and the
-// stage result written once.  Plane i+2 is fetched into registers at the top
-// of iteration i and stored to shared memory at its end, hiding the load
-// latency behind the flux work.  Domain-boundary faces take their outer state
+// stage result written once.  Plane i+2 (PPM: i+3) is asked for at the top of
+// iteration i, which hides its latency behind the flux work: in FP64 by asynchronous
+// copies into a ring slot of its own, in FP32 into registers that are converted and
+// stored to shared memory at the iteration's end.  Domain-boundary faces take their outer state
 // from the boundary pass (k_boundary), which applies the reference's interface
 // rules (src/bounCondOnInterfaces.c:11-110) to the reconstructed boundary cells.
 #pragma once
@@ -786,10 +787,11 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
                 if (!(base[0] > 0.0)) atomicOr(a.status, 2u);
             }
         }
-        // (g) plane i+2 into the ring slot of plane i (all readers of plane i
-        // passed the barrier above) and its velocities into the slots of
-        // planes i-1 (reciprocal ring) and i (division planes), read next
-        // after the next iteration's barrier; advance the march
+        // (g) FP32: plane i+2 (PPM: i+3) into the ring slot of plane i (PPM: i-1; all
+        // its readers passed the barrier above); FP64 planes are there already.  The
+        // velocities of plane i+2 into the slots of planes i-1 (reciprocal ring) and
+        // i (division planes), read next after the next iteration's barrier; advance
+        // the march
         if constexpr (PPM)
             plane_store<T, TJE, PPM>(s, SM::slot(i + 3), r, l, j, k, H, D, live && i + 3 <= L + 1, pl);
         else
@@ -827,7 +829,9 @@ __global__ void __launch_bounds__(TJE * 32, MINB) k_stage(Grid g, Consts kc, Arg
 // Parts of each march: as many as fill the SMs the grid's blocks leave idle, down
 // to two planes a part.  Used where no bit may change (the FP32 PPM tile).  Three
 // stages at 64x32x32 983 -> 172 us, 128x64x64 993 -> 395 us, 110x48x80 998 -> 333 us;
-// with more than half the SMs at work a second part has no SM to run on.
+// with more than half the SMs at work in the one wave a second part has no SM to run
+// on.  (Several waves are not cut, though the last may be uneven: 300 marches on 148 SMs
+// at 256x128x128 end after 100 planes where an even share is 90.)
 inline int march_split(const Grid &g, int nb, int seg, int sms)
 {
     return std::max(1, std::min(sms / nb, std::min(seg, g.L) / 2));

@@ -43,11 +43,11 @@ constexpr int WK = 32;           // tile columns (lanes)
 constexpr int NT = (3 * WJ + 3) * WK; // threads of a block: three groups and three halo warps
 
 struct Smem {
-    double U[4][WJ + 4][WK + 4][5];  // state of planes i .. i+3 (ring): rows -2..9, cols -2..33
-    double R[3][WJ + 2][WK + 2][3];  // velocities by reciprocal, planes i-1, i, i+1 (ring): rows -1..8, cols -1..32
+    double U[4][WJ + 4][WK + 4][5];  // state of planes i .. i+3 (ring): rows -2..5, cols -2..33
+    double R[3][WJ + 2][WK + 2][3];  // velocities by reciprocal, planes i-1, i, i+1 (ring): rows -1..4, cols -1..32
     double Dv[2][WJ + 2][WK + 2][5]; // velocities by division, T, face-averaged mu: planes i, i+1
     double K[2][WJ + 2][WK + 2][4];  // C, 1/(2C), 1/(2C)/C, |u|^2: planes i, i+1
-    double SL[3][WJ + 1][WK + 1][5]; // per direction, state on the face before each cell (row 8, column 32: halo)
+    double SL[3][WJ + 1][WK + 1][5]; // per direction, state on the face before each cell (row 4, column 32: halo)
     double SF[2][WJ + 1][WK + 1][5]; // y, z fluxes of the face before each cell
     double co[WJ];                   // Courant maxima, per warp of group x
 };
